@@ -60,12 +60,12 @@ typedef struct {
 /* Counters of one call (zeroed at the start of each call that fills them). */
 typedef struct {
   int64_t inverted_faces;        /* faces with orientation <= 0 after the move */
-  int64_t reverted_vertices;     /* vertices moved back while untangling */
-  int64_t removed_vertices;      /* vertices removed and reinserted */
+  int64_t reverted_vertices;     /* vertices moved back while untangling, or whose star it made anew */
+  int64_t removed_vertices;      /* vertices removed and reinserted, or whose star untangling made anew */
   int64_t lawson_flips;          /* Delaunay edge flips */
   int64_t lawson_rounds;         /* parallel flip rounds */
   int64_t removal_flips;         /* flips made while removing vertices */
-  int64_t insert_rounds;         /* parallel insertion rounds */
+  int64_t insert_rounds;         /* parallel insertion rounds, or rounds of stars */
   int64_t incircle_tests;        /* incircle evaluations */
   int64_t incircle_fp64;         /* ... that the FP32 filter could not decide */
   int64_t incircle_exact;        /* ... that the FP64 filter could not decide */
@@ -136,8 +136,9 @@ int mcl_integrate(mcl_mesh* m, const float* dt_dev, const mcl_float2* v_dev, voi
 
 /* untangle / untangle2 (include/Device_Triangulation.h:422-495).  Unlike the
  * reference (which only handles its B and C cases), this always returns a valid
- * triangulation: vertices of inverted faces are moved back, removed and
- * reinserted at their new positions, and the result is Delaunay. */
+ * triangulation: the vertices around the faces turned over get their stars anew
+ * at the new positions (or are moved back, removed and reinserted), and the
+ * result is Delaunay. */
 int mcl_untangle(mcl_mesh* m, void* stream, mcl_step_stats* stats_host);
 
 /* delonize / delonize2 (include/Device_Triangulation.h:324-390): Lawson flips to the

@@ -280,17 +280,19 @@ int mcl_batch_create(mcl_mesh* const* meshes, int64_t count, mcl_mesh** out) {
     return code;
   };
   if (cudaMalloc((void**)&b->vcomp, 4 * V) != cudaSuccess || cudaMalloc((void**)&b->vroot, 4 * V) != cudaSuccess ||
-      cudaMalloc((void**)&b->cbase, 4 * count) != cudaSuccess)
+      cudaMalloc((void**)&b->cbase, 4 * (count + 1)) != cudaSuccess ||
+      cudaMalloc((void**)&b->cebase, 4 * count) != cudaSuccess)
     return bail(fail(MCL_ERR_OUT_OF_MEMORY, "mcl_batch_create: component tables"));
   b->ncomp = count;
   b->comp_host = new int64_t[4 * count];
-  std::vector<int> base((size_t)count);
+  std::vector<int> base((size_t)count + 1), ebase((size_t)count);
   b->T = 0;
   int64_t vb = 0, eb = 0;
   for (int64_t i = 0; i < count; ++i) {
     mcl_mesh* m = meshes[i];
     b->comp_host[4 * i] = vb;
     base[(size_t)i] = (int)vb;
+    ebase[(size_t)i] = (int)eb;
     b->comp_host[4 * i + 1] = m->V;
     b->comp_host[4 * i + 2] = eb;
     b->comp_host[4 * i + 3] = m->E;
@@ -303,7 +305,9 @@ int mcl_batch_create(mcl_mesh* const* meshes, int64_t count, mcl_mesh** out) {
     vb += m->V;
     eb += m->E;
   }
-  if (cudaMemcpy(b->cbase, base.data(), 4 * count, cudaMemcpyHostToDevice) != cudaSuccess ||
+  base[(size_t)count] = (int)vb;
+  if (cudaMemcpy(b->cbase, base.data(), 4 * (count + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(b->cebase, ebase.data(), 4 * count, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaDeviceSynchronize() != cudaSuccess)
     return bail(fail(MCL_ERR_CUDA, "mcl_batch_create: sync"));
   b->dirty = new unsigned char[(size_t)count]();
@@ -361,10 +365,12 @@ int mcl_mesh_clone(const mcl_mesh* src, mcl_mesh** out) {
   if (e == cudaSuccess && src->vcomp) {
     e = cudaMalloc((void**)&m->vcomp, 4 * V);
     if (e == cudaSuccess) e = cudaMalloc((void**)&m->vroot, 4 * V);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&m->cbase, 4 * src->ncomp);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&m->cbase, 4 * (src->ncomp + 1));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&m->cebase, 4 * src->ncomp);
     if (e == cudaSuccess) e = cudaMemcpy(m->vcomp, src->vcomp, 4 * V, cudaMemcpyDeviceToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(m->vroot, src->vroot, 4 * V, cudaMemcpyDeviceToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(m->cbase, src->cbase, 4 * src->ncomp, cudaMemcpyDeviceToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(m->cbase, src->cbase, 4 * (src->ncomp + 1), cudaMemcpyDeviceToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(m->cebase, src->cebase, 4 * src->ncomp, cudaMemcpyDeviceToDevice);
   }
   if (e != cudaSuccess) {
     free_mesh(m);

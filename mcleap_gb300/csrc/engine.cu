@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "star.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -239,10 +240,26 @@ __device__ __forceinline__ void claim_edge(const KParams& P, int e, unsigned sc)
   claim_edge_with(P, e, ld_en(P, e), sc);
 }
 
+// The vertices of an edge that is not Delaunay or has a non-positive face: if
+// the step has a face to untangle, their stars are made anew (star.cuh).  Only
+// the step's first classification marks (kFixedPos): the removal path keeps its
+// own marks in vmark.
+template <bool kMark>
+__device__ __forceinline__ void mark_quad(const KParams& P, const int4 q, unsigned stamp) {
+  if (!kMark) return;
+  __stcg(P.vmark + q.x, (int)stamp);
+  __stcg(P.vmark + q.y, (int)stamp);
+  if (q.z >= 0) __stcg(P.vmark + q.z, (int)stamp);
+  if (q.w >= 0) __stcg(P.vmark + q.w, (int)stamp);
+}
+
 // Full predicate ladder for one edge: counts its non-positive faces into `bad`
 // and returns true when both faces are positive and the edge is non-Delaunay.
+// (An edge that is either marks the vertices of its quad and itself: `cand` is
+// the claim's stamp for one, set here for the other.)
 template <bool kFixedPos>
-__device__ __forceinline__ bool resolve_edge(const KParams& P, int e, LocalCounters& lc, int& bad) {
+__device__ __forceinline__ bool resolve_edge(const KParams& P, int e, unsigned qstamp, unsigned sc, LocalCounters& lc,
+                                             int& bad) {
   const int4 q = ld_ev(P, e);
   const float2 a = ldpos_t<kFixedPos>(P, q.x), b = ldpos_t<kFixedPos>(P, q.y);
   const float2 c = q.z >= 0 ? ldpos_t<kFixedPos>(P, q.z) : a;
@@ -251,11 +268,15 @@ __device__ __forceinline__ bool resolve_edge(const KParams& P, int e, LocalCount
   const int sb = q.w >= 0 ? orient_v(P, b, a, d, lc) : 1;
   if (sa <= 0 || sb <= 0) {
     bad += (sa <= 0) + (sb <= 0);
+    mark_quad<kFixedPos>(P, q, qstamp);
+    __stcg(P.cand + e, sc);
     return false;
   }
   if (q.z < 0 || q.w < 0) return false;
   lc.incircle++;
-  return incircle_sos(a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, q.x, q.y, q.z, q.w, &lc, &lc.overflow) > 0;
+  if (incircle_sos(a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, q.x, q.y, q.z, q.w, &lc, &lc.overflow) <= 0) return false;
+  mark_quad<kFixedPos>(P, q, qstamp);
+  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -298,10 +319,19 @@ constexpr int kMoveUnroll = 4;
 // of the thread itself and no block barrier is involved.  The first
 // iteration's records are requested before the move pass, which hides them.
 constexpr int kEvStages = 2;
-__shared__ int4 s_ev[kEvStages][kClassifyUnroll][kThreads];
-// the classification's append buffers (non-Delaunay edges, edges of a face
-// turned over): kWarpBuf entries per warp each
-__shared__ int s_wbuf[2][kThreads / 32][kWarpBuf];
+// Behind them the classification's append buffers (non-Delaunay edges, edges of
+// a face turned over): kWarpBuf entries per warp each.  One block of shared
+// memory, which the star phases use whole for their candidate lists.
+constexpr int kEvSlots = kEvStages * kClassifyUnroll * kThreads;
+constexpr int kPool = kEvSlots + 2 * (kThreads / 32) * kWarpBuf / 4;
+constexpr int kStarSlots = kPool / kThreads;  // candidates per thread in the pool
+__shared__ int4 s_pool[kPool];
+__device__ __forceinline__ int4* ev_slot(int stage, int j) {
+  return s_pool + (stage * kClassifyUnroll + j) * kThreads + threadIdx.x;
+}
+__device__ __forceinline__ int* warp_buf(int which) {
+  return reinterpret_cast<int*>(s_pool + kEvSlots) + (which * (kThreads / 32) + (threadIdx.x >> 5)) * kWarpBuf;
+}
 
 __device__ __forceinline__ void cp_async16(int4* smem, const int4* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -319,7 +349,7 @@ __device__ __forceinline__ void stage_edges(const KParams& P, int base, int st) 
 #pragma unroll
   for (int j = 0; j < kClassifyUnroll; ++j) {
     const int ei = base + j * blockDim.x + threadIdx.x;
-    if (ei < P.E_it) cp_async16(&s_ev[st][j][threadIdx.x], P.ev + edge_at(P, ei));
+    if (ei < P.E_it) cp_async16(ev_slot(st, j), P.ev + edge_at(P, ei));
   }
   cp_async_commit();
 }
@@ -363,7 +393,7 @@ __device__ void classify_one(const KParams& P, int e, unsigned qstamp, unsigned 
     return;
   }
   const int bad0 = bad;
-  if (resolve_edge<kFixedPos>(P, e, lc, bad) && enqueue_once(P, e, qstamp)) {
+  if (resolve_edge<kFixedPos>(P, e, qstamp, sc, lc, bad) && enqueue_once(P, e, qstamp)) {
     claim_edge(P, e, sc);
     push_one(P, P.wl0, &P.st->wl_count[0], e);
   }
@@ -385,8 +415,9 @@ __device__ void classify_movers(const KParams& P, int nm, unsigned qstamp, unsig
   warp_add(&P.st->inverted, bad);
 }
 
+// Returns whether only the movers' stars were classified.
 template <bool kFixedPos>
-__device__ void phase_classify(cg::grid_group& g, const KParams& P, unsigned qstamp, unsigned sc,
+__device__ bool phase_classify(cg::grid_group& g, const KParams& P, unsigned qstamp, unsigned sc,
                                LocalCounters& lc) {
   const int stride = gridDim.x * blockDim.x;
   constexpr int U = kClassifyUnroll;
@@ -437,13 +468,13 @@ __device__ void phase_classify(cg::grid_group& g, const KParams& P, unsigned qst
       cp_async_wait<0>();  // the prefetched records are not used
       classify_movers<kFixedPos>(P, nm, qstamp, sc, lc);
       if (kFixedPos) timeline_max(P, 45);
-      return;
+      return true;
     }
   }
   int bad = 0;
   unsigned ninc = 0;
   int def0 = -1, def1 = -1;  // edges deferred to the full ladder after the loop
-  WarpBuf wnd{s_wbuf[0][threadIdx.x >> 5], 0}, winv{s_wbuf[1][threadIdx.x >> 5], 0};
+  WarpBuf wnd{warp_buf(0), 0}, winv{warp_buf(1), 0};
   // kClassifyUnroll edges per thread and iteration, their records and
   // positions loaded before any is evaluated (memory-level parallelism: the
   // pass is latency-bound on the position gathers); edge j of the iteration
@@ -459,7 +490,7 @@ __device__ void phase_classify(cg::grid_group& g, const KParams& P, unsigned qst
     for (int j = 0; j < U; ++j) {
       const int ei = base + j * blockDim.x + threadIdx.x;
       e[j] = ei < P.E_it ? edge_at(P, ei) : -1;
-      q[j] = e[j] >= 0 ? s_ev[it % kEvStages][j][threadIdx.x] : make_int4(-1, -1, -1, -1);
+      q[j] = e[j] >= 0 ? *ev_slot(it % kEvStages, j) : make_int4(-1, -1, -1, -1);
     }
     float2 pa[U], pb[U], pc[U], pd[U];
 #pragma unroll
@@ -495,6 +526,8 @@ __device__ void phase_classify(cg::grid_group& g, const KParams& P, unsigned qst
         defer = true;
       } else if (sa <= 0 || sb <= 0) {
         bad += (sa <= 0) + (sb <= 0);
+        mark_quad<kFixedPos>(P, r, qstamp);
+        __stcg(P.cand + e[j], sc);
         inv[ki++] = e[j];
       } else if (r.z >= 0 && r.w >= 0) {
         ++ninc;
@@ -505,6 +538,7 @@ __device__ void phase_classify(cg::grid_group& g, const KParams& P, unsigned qst
           // each edge comes once in this pass and qstamp is the launch's
           // first stamp: the queue mark is a plain store (no atomic waited for)
           __stcg(P.qmark + e[j], qstamp);
+          mark_quad<kFixedPos>(P, r, qstamp);
           claim_edge(P, e[j], sc);
           mine[k++] = e[j];
         }
@@ -536,7 +570,7 @@ __device__ void phase_classify(cg::grid_group& g, const KParams& P, unsigned qst
       const int e = defs[j];
       if (e < 0) continue;
       const int bad0 = bad;
-      if (resolve_edge<kFixedPos>(P, e, lc, bad) && enqueue_once(P, e, qstamp)) {
+      if (resolve_edge<kFixedPos>(P, e, qstamp, sc, lc, bad) && enqueue_once(P, e, qstamp)) {
         claim_edge(P, e, sc);
         mine[k++] = e;
       }
@@ -548,6 +582,7 @@ __device__ void phase_classify(cg::grid_group& g, const KParams& P, unsigned qst
   lc.incircle += ninc;
   warp_add(&P.st->inverted, bad);
   if (kFixedPos) timeline_max(P, 45);
+  return false;
 }
 
 // Resolve the hard list of phase_classify (after its barrier) with the full
@@ -569,7 +604,7 @@ __device__ void phase_classify_hard(cg::grid_group& g, const KParams& P, unsigne
     if (i < n) {
       const int e = ld_i(P.hard + i);
       const int bad0 = bad;
-      if (resolve_edge<kFixedPos>(P, e, lc, bad) && enqueue_once(P, e, qstamp)) {
+      if (resolve_edge<kFixedPos>(P, e, qstamp, sc, lc, bad) && enqueue_once(P, e, qstamp)) {
         claim_edge(P, e, sc);
         mine[k++] = e;
       }
@@ -624,7 +659,7 @@ __device__ __forceinline__ int lawson_round(const KParams& P, const int* in, int
   }
   int flips = 0;
   const int lane = threadIdx.x & 31;
-  WarpBuf wb{s_wbuf[0][threadIdx.x >> 5], 0};
+  WarpBuf wb{warp_buf(0), 0};
   for (int base = t0 - lane; base < n; base += nt) {
     const int i = base + lane;
     int mine[4];
@@ -869,7 +904,7 @@ __device__ bool phase_fixpoint(cg::grid_group& g, const KParams& P, LocalCounter
       // warp's append buffers, idle after the classification)
       const int nb = ld_i(&P.st->wl_count[1]);
       const int lane = threadIdx.x & 31;
-      WarpBuf whard{s_wbuf[0][threadIdx.x >> 5], 0}, wnext{s_wbuf[1][threadIdx.x >> 5], 0};
+      WarpBuf whard{warp_buf(0), 0}, wnext{warp_buf(1), 0};
       int* nlist = (pass & 1) ? P.vl1 : P.vl0;
       int* ncount = &P.st->fix_list[pass % 3];
       for (int base = spread_tid() - lane; base < nb; base += stride) {
@@ -972,7 +1007,7 @@ constexpr int kSmallStar = 16;
 struct SmallPoly {
   unsigned long long nx_ = 0, pv_ = 0;
   __device__ __forceinline__ static float2* slot(int j) {
-    return reinterpret_cast<float2*>(&s_ev[(j >> 3) & 1][(j >> 1) & 3][threadIdx.x]) + (j & 1);
+    return reinterpret_cast<float2*>(ev_slot((j >> 3) & 1, (j >> 1) & 3)) + (j & 1);
   }
   __device__ __forceinline__ int nx(int j) const { return (int)((nx_ >> (4 * j)) & 15u); }
   __device__ __forceinline__ int pv(int j) const { return (int)((pv_ >> (4 * j)) & 15u); }
@@ -1395,7 +1430,7 @@ __device__ bool phase_remove(cg::grid_group& g, const KParams& P, unsigned& stam
     if (round < 16) timeline_remove(P, 4 * round + 1);
     int removed = 0, flips = 0;
     unsigned long long slow = 0;  // the slowest removal of this thread: cycles << 16 | spokes
-    WarpBuf wb{s_wbuf[0][threadIdx.x >> 5], 0};
+    WarpBuf wb{warp_buf(0), 0};
     for (int base = wid * T; base < n; base += di) {
       const int i = lane < T ? base + lane : n;
       int mine[1];
@@ -1677,7 +1712,7 @@ __device__ bool phase_insert(cg::grid_group& g, const KParams& P, unsigned& stam
     g.sync();
     timeline_insert(P, round, 1);
     int inserted = 0;
-    WarpBuf wagain{s_wbuf[1][threadIdx.x >> 5], 0};
+    WarpBuf wagain{warp_buf(1), 0};
     for (int base = spread_tid() - (int)(threadIdx.x & 31); base < n; base += stride) {
       const int i = base + (int)(threadIdx.x & 31);
       int mine[8];
@@ -1804,6 +1839,9 @@ __device__ void finish_launch(const KParams& P, unsigned stamp) {
   st->inverted = 0;
   st->hard_count = 0;
   for (int i = 0; i < 3; ++i) st->fix_new[i] = st->fix_bad[i] = st->fix_list[i] = 0;
+  for (int i = 0; i < 3; ++i) st->star_n[i] = 0;
+  st->star_ext = 0;
+  st->star_made = 0;
   st->fix_all = 0;
   st->mark_ovf = 0;
   st->movers_last = __ldcg(&st->movers_now);
@@ -2051,7 +2089,7 @@ __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, 
     if (gtid == 0) { P.st->vl_count[0] = 0; P.st->vl_count[1] = 0; }
     g.sync();
     const int nsb = few ? nall : P.V_it;
-    WarpBuf wrev{s_wbuf[0][threadIdx.x >> 5], 0};
+    WarpBuf wrev{warp_buf(0), 0};
     for (int base = (few ? spread_tid() - (int)(threadIdx.x & 31) : blockIdx.x * blockDim.x); base < nsb;
          base += stride) {
       const int vi = base + (few ? (int)(threadIdx.x & 31) : (int)threadIdx.x);
@@ -2112,7 +2150,7 @@ __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, 
       // else by a pass over the vertices
       const bool from_list = few && !(nrev > 0 && P.substeps > 0);
       const int nscan = from_list ? nall : P.V_it;
-      WarpBuf wins{s_wbuf[0][threadIdx.x >> 5], 0};
+      WarpBuf wins{warp_buf(0), 0};
       for (int base = (from_list ? spread_tid() - (int)(threadIdx.x & 31) : blockIdx.x * blockDim.x); base < nscan;
            base += stride) {
         const int vi = base + (from_list ? (int)(threadIdx.x & 31) : (int)threadIdx.x);
@@ -2144,7 +2182,7 @@ __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, 
       if (rebuild) {
         if (gtid == 0) { P.st->wl_count[0] = 0; P.st->wl_count[1] = 0; }
         g.sync();
-        WarpBuf wb{s_wbuf[0][threadIdx.x >> 5], 0};
+        WarpBuf wb{warp_buf(0), 0};
         for (int base = blockIdx.x * blockDim.x; base < P.E_it; base += stride) {
           const int ei = base + threadIdx.x;
           const int e = ei < P.E_it ? edge_at(P, ei) : -1;
@@ -2160,7 +2198,7 @@ __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, 
         const unsigned du = stamp++;  // first sight of an edge in this pass (cand is free until the flip rounds)
         if (gtid == 0) P.st->wl_count[1] = 0;
         g.sync();
-        WarpBuf wb{s_wbuf[0][threadIdx.x >> 5], 0};
+        WarpBuf wb{warp_buf(0), 0};
         for (int base = spread_tid() - (int)(threadIdx.x & 31); base < nw; base += stride) {
           const int i = base + (int)(threadIdx.x & 31);
           int mine[1];
@@ -2184,22 +2222,622 @@ __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, 
   return stamp;
 }
 
+// ---------------------------------------------------------------------------
+// Untangling by stars (star.cuh) inside the step's launch.
+
+// A vertex's candidates in this thread's slots of the shared pool (idle after
+// the classification).
+struct SharedCand {
+  MCL_HD int cap() const { return kStarSlots; }
+  __device__ __forceinline__ static float4* at(int i) {
+    return reinterpret_cast<float4*>(s_pool) + i * kThreads + threadIdx.x;
+  }
+  __device__ __forceinline__ Cand get(int i) const {
+    const float4 q = *at(i);
+    return Cand{q.x, q.y, q.z, __float_as_int(q.w)};
+  }
+  __device__ __forceinline__ void set(int i, Cand c) { *at(i) = make_float4(c.x, c.y, c.key, __int_as_float(c.id)); }
+};
+
+// The same for any number of candidates, in local memory: the vertices that
+// neither the pool's slots nor a warp can take.
+__device__ __noinline__ int star_wide(const KParams& P, int v, bool keep, unsigned bad, bool again,
+                                      LocalCounters* lc) {
+  LocalCand L;
+  return again ? star_from_stars(P, v, L, *lc) : star_from_mesh(P, v, keep, bad, L, *lc);
+}
+__device__ __forceinline__ bool star_alone(const KParams& P, int v, bool keep, unsigned bad, bool again,
+                                           LocalCounters& lc) {
+  LocalCounters m = {0, 0, 0, 0, 0, 0, 0};
+  const int rc = star_wide(P, v, keep, bad, again, &m);
+  star_count(lc, m);
+  return rc == kStarOk;
+}
+
+// ---- one warp per vertex, one candidate (or neighbour) per lane ----------------
+// A lone thread takes tens of microseconds over a star (a thousand dependent
+// instructions); a warp takes a few.  Each returns false, having written nothing,
+// where the thread's form has to decide: wide or open stars, candidates on (nearly)
+// one ray, anything malformed.
+
+// The star from candidate x of each lane that has one.
+__device__ __forceinline__ bool warp_star(const KParams& P, int v, MeshBase mb, int x, bool valid,
+                                          LocalCounters& lc) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const float2 pv = P.pos[v];
+  float4* slot = reinterpret_cast<float4*>(s_pool) + (threadIdx.x & ~31);
+  auto at = [&](int i) {
+    const float4 q = slot[i];
+    return Cand{q.x, q.y, q.z, __float_as_int(q.w)};
+  };
+  unsigned alive = 0;
+  int p = 0, s = 0;
+  auto beside = [&] {
+    const unsigned below = alive & lt, above = alive & ~lt & ~(1u << lane);
+    p = 31 - __clz(below ? below : alive);
+    s = __ffs(above ? above : alive) - 1;
+  };
+  Cand c;
+  unsigned live = __ballot_sync(kFull, valid);
+  if (valid) valid = __ffs(__match_any_sync(live, x)) - 1 == lane;  // one lane per vertex
+  bool open = true;
+  for (int pass = 0; pass < 2 && open; ++pass) {
+    if (pass) {
+      // the fan does not close: the corners join (none of them is in a lane yet,
+      // or the lane that has it stays)
+      const unsigned free = ~__ballot_sync(kFull, valid);
+      if (__popc(free) < 4) return false;
+      const int k = __popc(free & lt);
+      if ((free >> lane & 1u) && k < 4) {
+        x = mb.v0 + k;
+        valid = true;
+      }
+      live = __ballot_sync(kFull, valid);
+      if (valid) valid = __ffs(__match_any_sync(live, x)) - 1 == lane;
+    }
+    c = valid ? star_cand(pv, x, P.pos[x], 0.f) : Cand{0.f, 0.f, 0.f, -1};
+    if (__any_sync(kFull, valid && !(c.key >= 0.f))) return false;
+    live = __ballot_sync(kFull, valid);
+    if (__popc(live) < 3) continue;
+    const float from = __shfl_sync(kFull, c.key, __ffs(live) - 1);
+    c.key -= from;
+    if (c.key < 0.f) c.key += 4.f;
+    // place in the angular order; of two on one ray the farther leaves
+    int rank = 0;
+    for (;;) {
+      rank = 0;
+      bool out = false, same = false;
+      for (unsigned m = live; m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const float kj = __shfl_sync(kFull, c.key, j);
+        bool before = kj < c.key;
+        const bool near = valid && j != lane && fabsf(kj - c.key) < kStarSameKey;
+        if (__any_sync(kFull, near)) {
+          Cand u;
+          u.x = __shfl_sync(kFull, c.x, j);
+          u.y = __shfl_sync(kFull, c.y, j);
+          u.id = __shfl_sync(kFull, c.id, j);
+          if (near) {
+            int r = star_cross(u, c);
+            if (r == 2) {
+              LocalCounters t = {0, 0, 0, 0, 0, 0, 0};
+              r = star_cross_exact(P.pos, v, u.id, c.id, &t);
+              star_count(lc, t);
+              if (r == 0) {
+                const int nearer = star_nearer(P.pos, v, u.id, c.id);
+                same |= nearer < 0;
+                out |= nearer == 0;
+              }
+            }
+            before = r > 0;
+          }
+          __syncwarp();
+        }
+        rank += before ? 1 : 0;
+      }
+      if (__any_sync(kFull, same)) return false;
+      if (!__any_sync(kFull, out)) break;
+      valid = valid && !out;
+      live = __ballot_sync(kFull, valid);
+    }
+    const int n = __popc(live);
+    __syncwarp();
+    if (valid) slot[rank] = make_float4(c.x, c.y, c.key, __int_as_float(c.id));
+    __syncwarp();
+    alive = n == 32 ? kFull : (1u << n) - 1u;
+    c = at(lane < n ? lane : 0);
+    // every lane tests its candidate against the two beside it; of two neighbours
+    // that would drop only the first does, so what drops is redundant among those
+    // that stay
+    for (int turn = 0; turn < 64 && __popc(alive) > 3; ++turn) {
+      const bool in = alive >> lane & 1u;
+      beside();
+      int r = 0;
+      if (in) {
+        const Cand a = at(p), b = at(s);
+        r = star_cross(a, b);
+        if (r == 1) {
+          lc.incircle++;
+          r = star_outside(a, b, c);
+        }
+        if (r == 2) {
+          LocalCounters t = {0, 0, 0, 0, 0, 0, 0};
+          r = star_cross_exact(P.pos, v, a.id, b.id, &t);
+          if (r > 0) r = star_outside_exact(P.pos, v, a.id, b.id, c.id, &t);
+          star_count(lc, t);
+        }
+      }
+      __syncwarp();
+      const unsigned d = __ballot_sync(kFull, in && r > 0);
+      if (!d) break;
+      unsigned rm = __ballot_sync(kFull, (d >> lane & 1u) && !(d >> p & 1u));
+      if (!rm) rm = d & (0u - d);
+      alive &= ~rm;
+    }
+    beside();
+    bool gap = false;
+    if (alive >> lane & 1u) {
+      const Cand b = at(s);
+      int r = star_cross(c, b);
+      if (r == 2) {
+        LocalCounters t = {0, 0, 0, 0, 0, 0, 0};
+        r = star_cross_exact(P.pos, v, c.id, b.id, &t);
+        star_count(lc, t);
+      }
+      gap = r <= 0;
+    }
+    open = __any_sync(kFull, gap);
+    if (open) {  // what has dropped stays redundant when the corners join
+      valid = alive >> lane & 1u;
+      x = c.id;
+    }
+  }
+  const int k = __popc(alive);
+  if (open || k < 3 || k > kRowInline) return false;
+  const bool in = alive >> lane & 1u;
+  const int i = __popc(alive & lt);
+  const int own = __reduce_or_sync(kFull, in && star_owned(v, c.id, mb.v0 + 4) ? 1u << i : 0u);
+  int* row = P.srow + (size_t)v * kRow;
+  if (in) __stcg(row + 1 + i, c.id);
+  if (lane == 0) __stcg(row, k | own << kRowOwn);
+  return true;
+}
+
+__device__ __forceinline__ bool warp_from_mesh(const KParams& P, int v, bool keep, unsigned bad, LocalCounters& lc) {
+  const int lane = threadIdx.x & 31, HE = 2 * P.E;
+  const MeshBase mb = star_base(P, v);
+  const int s0 = P.vhe[v];
+  if ((unsigned)s0 >= (unsigned)HE) return false;
+  int h = s0, k = 0, mine = 0;
+  do {  // the ring: every lane walks, lane k keeps the k-th side
+    const int4 r = P.en[h >> 1];
+    const int nx = (h & 1) ? r.z : r.x, pr = (h & 1) ? r.w : r.y;
+    if ((unsigned)nx >= (unsigned)HE || (unsigned)pr >= (unsigned)HE) return false;
+    if (lane == k) mine = nx;
+    ++k;
+    h = pr ^ 1;
+  } while (h != s0 && k < 16);
+  if (h != s0 || k > kRowInline) return false;
+  int x = -1, o = -1;
+  bool fine = true;
+  if (lane < k) {
+    const int4 e = P.ev[mine >> 1];
+    const bool across = !keep && P.cand[mine >> 1] == bad;
+    x = (mine & 1) ? e.y : e.x;
+    o = (mine & 1) ? e.z : e.w;
+    fine = x >= mb.v0 && x < mb.v1 && o < mb.v1 && x != v;
+    if (!across || o < mb.v0 || o == v) o = -1;
+  }
+  if (!__all_sync(kFull, fine)) return false;
+  if (keep) {
+    const int own = __reduce_or_sync(kFull, lane < k && star_owned(v, x, mb.v0 + 4) ? 1u << lane : 0u);
+    int* row = P.srow + (size_t)v * kRow;
+    if (lane < k) __stcg(row + 1 + lane, x);
+    if (lane == 0) __stcg(row, k | own << kRowOwn);
+  } else {
+    const int far = __shfl_sync(kFull, o, lane & 15);
+    if (lane >= 16) x = far;
+    if (!warp_star(P, v, mb, x, x >= 0, lc)) return false;
+  }
+  if (lane == 0) __stcg(P.sinbox + (size_t)kInbox * v, 0);
+  return true;
+}
+
+__device__ __forceinline__ bool warp_from_stars(const KParams& P, int v, LocalCounters& lc) {
+  const int lane = threadIdx.x & 31;
+  const MeshBase mb = star_base(P, v);
+  const int* row = P.srow + (size_t)v * kRow;
+  int* box = P.sinbox + (size_t)kInbox * v;
+  const int h = row[0], n = h & kRowCount, m = min(box[0], kInbox - 1);
+  if ((h & (kRowExt | kRowOpen)) || n > kRowInline) return false;
+  const int x = lane < n ? row[1 + lane] : (lane < n + m ? box[1 + lane - n] : -1);
+  const bool valid = lane < n + m;
+  if (!__all_sync(kFull, !valid || (x >= mb.v0 && x < mb.v1 && x != v))) return false;
+  if (!warp_star(P, v, mb, x, valid, lc)) return false;
+  if (lane == 0) __stcg(box, 0);
+  return true;
+}
+
+// star_check and star_commit, an entry per lane.
+template <typename Mark>
+__device__ __forceinline__ int warp_check(const KParams& P, int v, int c4, bool all, Mark mark, int* inner,
+                                          unsigned long long* ranks) {
+  const int lane = threadIdx.x & 31;
+  const int* row = P.srow + (size_t)v * kRow;
+  const int h = row[0], n = h & kRowCount;
+  *inner = 0;
+  *ranks = 0;
+  if ((h & kRowExt) || n > kRowInline || n < 3) {
+    int own = 0;
+    if (lane == 0) own = star_check(P, v, c4, all, mark, inner, ranks);
+    __syncwarp();
+    return own;  // lane 0's counts, and only its
+  }
+  const int w = lane < n ? row[1 + lane] : -1;
+  const int bf = __shfl_sync(kFull, w, lane ? lane - 1 : n - 1), af = __shfl_sync(kFull, w, lane + 1 < n ? lane + 1 : 0);
+  int r = 0, in = 0;
+  if (lane < n) {
+    const int4* theirs = reinterpret_cast<const int4*>(P.srow + (size_t)w * kRow);
+    r = star_check_entry(P, v, w, bf, af, c4, all, theirs[0], theirs[1], mark);
+    in = w >= c4 ? (star_owned(v, w, c4) ? 1 : -1) : 0;
+  }
+  __syncwarp();
+  const bool bad = __any_sync(kFull, r < 0) || (h & kRowOpen);
+  const unsigned q = (unsigned)min(r < 0 ? 0 : r, 15);
+  const unsigned lo = __reduce_or_sync(kFull, lane < 8 ? q << (4 * lane) : 0u);
+  const unsigned hi = __reduce_or_sync(kFull, lane >= 8 && lane < 15 ? q << (4 * (lane - 8)) : 0u);
+  in = __reduce_add_sync(kFull, in);
+  if (lane == 0) {
+    if (bad) mark(v);
+    *inner = in;
+    *ranks = (unsigned long long)hi << 32 | lo;
+    return __popc((unsigned)h >> kRowOwn & 0x7fffu);
+  }
+  return 0;
+}
+
+__device__ __forceinline__ bool warp_commit(const KParams& P, int v) {
+  const int lane = threadIdx.x & 31;
+  const int* row = P.srow + (size_t)v * kRow;
+  const int hd = row[0], n = hd & kRowCount;
+  bool fine = true;
+  if ((hd & kRowExt) || n > kRowInline) {
+    if (lane == 0) fine = star_commit(P, v);
+  } else {
+    const MeshBase mb = star_base(P, v);
+    const int w = lane < n ? row[1 + lane] : -1;
+    const int prev = lane ? lane - 1 : n - 1, next = lane + 1 < n ? lane + 1 : 0;
+    const int bf = __shfl_sync(kFull, w, prev), af = __shfl_sync(kFull, w, next);
+    const int mine = __popc((unsigned)hd >> kRowOwn & ((1u << min(lane, 15)) - 1u));
+    int h = 0;
+    if (lane < n) h = star_spoke(P, mb, v, w, lane, star_edge0(P, mb, v), mine, false, P.srank[v]);
+    __syncwarp();
+    const int hb = __shfl_sync(kFull, h, prev), ha = __shfl_sync(kFull, h, next);
+    if (!__all_sync(kFull, (unsigned)h < (unsigned)(2 * P.E))) return false;
+    if (lane < n) fine = star_put(P, mb, v, w, bf, af, h, hb, ha);
+    if (lane == 0) __stcg(P.vhe + v, h);
+  }
+  return __all_sync(kFull, fine);
+}
+
+// v and the vertices of its row get the stamp: their checks may come out
+// differently once v's row changes.
+__device__ __forceinline__ void warp_touch(const KParams& P, int v, unsigned stamp) {
+  const int lane = threadIdx.x & 31;
+  const int* row = P.srow + (size_t)v * kRow;
+  const int h = ld_i(row);
+  int n = h & kRowCount;
+  const int* at = row + 1;
+  if (h & kRowExt) {
+    const int e = ld_i(row + 1);
+    at = star_ext(P, e >= 0 && e < star_ext_rows(P.V) ? e : 0);
+    n = min(n, kExtRow);
+  } else {
+    n = min(n, kRowInline);
+  }
+  for (int i = lane; i < n; i += 32) {
+    const int w = ld_i(at + i);
+    if ((unsigned)w < (unsigned)P.V) __stcg(P.vaux + w, (int)stamp);
+  }
+  if (lane == 0) __stcg(P.vaux + v, (int)stamp);
+}
+
+// Sums of per-thread values over the block, in every thread.
+template <int N>
+__device__ __forceinline__ void block_sum(int (&x)[N]) {
+  __shared__ int part[N][kThreads / 32];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int y = __reduce_add_sync(kFull, x[k]);
+    if ((threadIdx.x & 31) == 0) part[k][threadIdx.x >> 5] = y;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    int y = 0;
+    for (int w = 0; w < kThreads / 32; ++w) y += part[k][w];
+    x[k] = y;
+  }
+}
+
+// A vertex whose star disagrees joins the round's list once.  Threads that
+// arrive together share one atomicAdd.
+constexpr int kStarGivenUp = 1 << 30;
+__device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, int* list, int* count) {
+  if (atomicMax(P.smark + u, cs) >= cs) return;
+  cg::coalesced_group grp = cg::coalesced_threads();
+  int base = 0;
+  if (grp.thread_rank() == 0) base = atomicAdd(count, (int)grp.size());
+  const int at = grp.shfl(base, 0) + (int)grp.thread_rank();
+  if (at < P.V) __stcg(list + at, u);
+}
+
+// A step that moved few vertices of a mesh larger than this is left to the removal
+// path, whose cost goes with the movers; the stars' goes with the mesh.
+constexpr int kStarSparse = 200000;
+
+// Vertices (or list entries) per warp of the launch up to which a warp takes one
+// vertex at a time; above it a thread does.
+constexpr int kWarpStars = 8;
+
+// Each block takes a run of consecutive vertices (their rows and positions meet
+// in its L1).  Returns false, with the mesh untouched, when the stars cannot be
+// made to agree.  A count is read by all threads after a barrier and next written
+// two barriers later, so all take the same branches; bit 30 of the next count says
+// that a star could not be made.
+__device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, unsigned& stamp, unsigned q0,
+                                          unsigned sc0, LocalCounters& lc) {
+  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = stride >> 5, gwarp = spread_tid() >> 5;
+  const int per = (P.V_it + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int i0 = min(P.V_it, (int)blockIdx.x * per), i1 = min(P.V_it, i0 + per);
+  const bool few = P.V_it <= kWarpStars * nwarps;
+  int* const cnt = P.st->star_n;
+  int* const lists[2] = {P.vl0, P.vl1};
+  int made = 0;
+  bool fine = true;
+  __syncthreads();  // the pool's last readers are done
+  if (few) {
+    for (int i = i0 + warp; i < i1; i += kThreads / 32) {
+      const int v = vert_at(P, i);
+      if (P.vfix[v]) continue;
+      const bool keep = (unsigned)ld_i(P.vmark + v) != q0;
+      if (lane == 0) made += keep ? 0 : 1;
+      if (!warp_from_mesh(P, v, keep, sc0, lc) && lane == 0) fine = star_alone(P, v, keep, sc0, false, lc) && fine;
+      __syncwarp();
+    }
+  } else {
+    for (int base = i0 + warp * 32; base < i1; base += kThreads) {
+      const int v = base + lane < i1 ? vert_at(P, base + lane) : -1;
+      const bool keep = v >= 0 && (unsigned)ld_i(P.vmark + v) != q0;
+      int rc = kStarOk;
+      if (v >= 0 && !P.vfix[v]) {
+        SharedCand L;
+        made += keep ? 0 : 1;
+        rc = star_from_mesh(P, v, keep, sc0, L, lc);
+      }
+      fine = fine && rc != kStarDegenerate;
+      // those with more candidates than the slots, by the whole warp
+      for (unsigned m = __ballot_sync(kFull, rc == kStarFull); m; m &= m - 1) {
+        const int j = __ffs(m) - 1, u = __shfl_sync(kFull, v, j);
+        const bool k = __shfl_sync(kFull, (int)keep, j) != 0;
+        if (!warp_from_mesh(P, u, k, sc0, lc) && lane == 0) fine = star_alone(P, u, k, sc0, false, lc) && fine;
+        __syncwarp();
+      }
+    }
+  }
+  __syncwarp();
+  warp_add(&P.st->star_made, made);
+  if (!fine) atomicOr(cnt, kStarGivenUp);
+  g.sync();
+  timeline(P, 43);
+  int slot = 0, rounds = 0;
+  int sums[4];
+  bool both = false;     // both ends of an edge look for each other
+  unsigned touched = 0;  // stamp of the vertices whose check may have changed (0: all)
+  for (;;) {
+    // every edge against its owner's row; own edges counted per vertex and block
+    unsigned cs = stamp++;
+    if (gtid == 0) cnt[(slot + 1) % 3] = 0;
+    sums[0] = sums[1] = sums[2] = sums[3] = 0;
+    auto mark = [&](int u) {
+      sums[3] = 1;
+      __stcg(P.smark + u, cs);
+    };
+    for (int i = i0 + (few ? warp : (int)threadIdx.x); i < i1; i += few ? kThreads / 32 : kThreads) {
+      const int v = vert_at(P, i);
+      int own = 0;
+      if (!P.vfix[v]) {
+        const int v0 = star_base(P, v).v0;
+        int inner;
+        unsigned long long ranks;
+        // after a round of few vertices only those whose rows met theirs have
+        // changed; the others keep what the last check found
+        const bool old = touched && (unsigned)ld_i(P.vaux + v) != touched;
+        if (old) {
+          const int w = ld_i(P.vlocf + v);
+          own = w & 0xffff;
+          inner = (w >> 16) - 128;
+        } else {
+          own = few ? warp_check(P, v, v0 + 4, both, mark, &inner, &ranks)
+                    : star_check(P, v, v0 + 4, both, mark, &inner, &ranks);
+        }
+        if (!few || lane == 0) {
+          if (!old) {
+            __stcg(P.srank + v, ranks);
+            __stcg(P.vlocf + v, own | (inner + 128) << 16);
+          }
+          sums[1] += own - 3 - (v == v0 + 4 ? 1 : 0);
+          sums[2] += inner;
+        }
+      } else if (!few || lane == 0) {
+        __stcg(P.vlocf + v, 0);
+      }
+      if (!few || lane == 0) sums[0] += own;
+    }
+    __syncwarp();
+    block_sum(sums);
+    if (threadIdx.x < 4) {
+      int x = sums[0];
+#pragma unroll
+      for (int k = 1; k < 4; ++k) x = threadIdx.x == k ? sums[k] : x;
+      __stcg(P.sblk + 4 * blockIdx.x + threadIdx.x, x);
+    }
+    g.sync();
+    if (ld_i(cnt + slot % 3) & kStarGivenUp) return false;
+    // own edges of the blocks before this one; the balance over all of them
+    sums[0] = sums[1] = sums[2] = sums[3] = 0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads) {
+      const int4 q = __ldcg(reinterpret_cast<const int4*>(P.sblk) + b);
+      if (b < (int)blockIdx.x) sums[0] += q.x;
+      sums[1] += q.y;
+      sums[2] += q.z;
+      sums[3] += q.w;
+    }
+    block_sum(sums);
+    if (sums[3] == 0) {
+      if (sums[1] == 0 && sums[2] == 0) break;
+      // an owner holds a vertex that does not hold it: look from both ends
+      if (both) return false;
+      both = true;
+      touched = 0;
+      ++slot;
+      g.sync();  // the sums have been read
+      continue;
+    }
+    // the marked vertices, listed in order
+    {
+      WarpBuf wb{warp_buf(0), 0};
+      for (int base = i0 + (int)(threadIdx.x & ~31); base < i1; base += kThreads) {
+        const int i = base + lane;
+        const int v = i < i1 ? vert_at(P, i) : 0;
+        const int mine[1] = {v};
+        const int k = i < i1 && (unsigned)ld_i(reinterpret_cast<const int*>(P.smark) + v) == cs ? 1 : 0;
+        if (__any_sync(kFull, k)) wb_push(wb, mine, k, lists[slot & 1], cnt + slot % 3, P.V, P.st);
+      }
+      wb_flush(wb, lists[slot & 1], cnt + slot % 3, P.V, P.st);
+    }
+    g.sync();
+    int n = ld_i(cnt + slot % 3);
+    if (n > kWarpStars * nwarps) {
+      // many stars disagree: a thread makes one, then everything is checked
+      if (++rounds > kStarRounds) return false;
+      fine = true;
+      for (int base = gwarp * 32; base < n; base += stride) {
+        const int v = base + lane < n ? ld_i(lists[slot & 1] + base + lane) : -1;
+        int rc = kStarOk;
+        if (v >= 0) {
+          SharedCand L;
+          rc = star_from_stars(P, v, L, lc);
+        }
+        fine = fine && rc != kStarDegenerate;
+        for (unsigned m = __ballot_sync(kFull, rc == kStarFull); m; m &= m - 1) {
+          const int u = __shfl_sync(kFull, v, __ffs(m) - 1);
+          if (!warp_from_stars(P, u, lc) && lane == 0) fine = star_alone(P, u, false, 0, true, lc) && fine;
+          __syncwarp();
+        }
+      }
+      if (!fine) atomicOr(cnt + (slot + 1) % 3, kStarGivenUp);
+      g.sync();
+      if (rounds <= 40) timeline(P, 1 + rounds);
+      touched = 0;
+      ++slot;
+      continue;
+    }
+    // few do: a warp makes one, then they check their neighbourhoods, until all agree
+    touched = stamp++;
+    while (n > 0) {
+      if (++rounds > kStarRounds) return false;
+      fine = true;
+      for (int i = gwarp; i < n; i += nwarps) {
+        const int v = ld_i(lists[slot & 1] + i);
+        warp_touch(P, v, touched);
+        if (!warp_from_stars(P, v, lc) && lane == 0) fine = star_alone(P, v, false, 0, true, lc) && fine;
+        __syncwarp();
+        warp_touch(P, v, touched);
+      }
+      if (!fine) atomicOr(cnt + (slot + 1) % 3, kStarGivenUp);
+      g.sync();
+      ++slot;
+      cs = stamp++;
+      if (gtid == 0) cnt[(slot + 1) % 3] = 0;
+      auto again = [&](int u) { star_list(P, u, cs, lists[slot & 1], cnt + slot % 3); };
+      for (int i = gwarp; i < n; i += nwarps) {
+        const int v = ld_i(lists[(slot - 1) & 1] + i);
+        int inner;
+        unsigned long long ranks;
+        warp_check(P, v, star_base(P, v).v0 + 4, true, again, &inner, &ranks);
+      }
+      __syncwarp();
+      g.sync();
+      if (rounds <= 40) timeline(P, 1 + rounds);
+      n = ld_i(cnt + slot % 3);
+      if (n >= kStarGivenUp || n < 0) return false;
+    }
+    ++slot;
+  }
+  timeline(P, 44);
+  int carry = sums[0];
+  __shared__ int wsum[kThreads / 32];
+  for (int base = i0; base < i1; base += kThreads) {
+    const int i = base + threadIdx.x;
+    const int v = i < i1 ? vert_at(P, i) : 0;
+    const int own = i < i1 ? ld_i(P.vlocf + v) & 0xffff : 0;
+    int x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, x, o);
+      if (lane >= o) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (w < warp) before += wsum[w];
+      all += wsum[w];
+    }
+    if (i < i1) __stcg(P.sbase + v, carry + before + x - own);
+    carry += all;
+  }
+  g.sync();
+  timeline(P, 45);
+  for (int i = i0 + (few ? warp : (int)threadIdx.x); i < i1; i += few ? kThreads / 32 : kThreads) {
+    const int v = vert_at(P, i);
+    if (P.vfix[v]) continue;
+    if (!(few ? warp_commit(P, v) : star_commit(P, v))) set_error(P, MCL_ERR_DEGENERATE_INPUT);
+  }
+  if (gtid == 0) {
+    P.st->c[C_INVERTED] += (unsigned long long)ld_i(&P.st->inverted);
+    const unsigned long long m = (unsigned long long)ld_i(&P.st->star_made);
+    P.st->c[C_REVERTED] += m;
+    P.st->c[C_REMOVED] += m;
+    P.st->c[C_INSERT_ROUNDS] += (unsigned long long)rounds + 1;
+  }
+  timeline(P, 46);
+  return true;
+}
+
 // One kinetic step in one persistent launch: (move +) classify; if a face is
-// inverted, repair; then Lawson rounds to the Delaunay triangulation.
-__global__ void __launch_bounds__(kThreads, 3) k_step(KParams P) {
+// inverted, untangle by stars, or, where that cannot be, by removal; else Lawson
+// rounds to the Delaunay triangulation.
+__global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KParams P) {
   cg::grid_group g = cg::this_grid();
   LocalCounters lc = {0, 0, 0, 0, 0, 0, 0};
   unsigned stamp = ld_i(reinterpret_cast<const int*>(&P.st->epoch));
   timeline(P, 0);
   const unsigned q0 = stamp++;
   const unsigned sc0 = stamp++;
-  phase_classify<true>(g, P, q0, sc0, lc);
+  const bool sparse = phase_classify<true>(g, P, q0, sc0, lc);
   g.sync();
   phase_classify_hard<true>(g, P, q0, sc0, lc);
   timeline(P, 1);
   const int inverted = ld_i(&P.st->inverted);
   if (inverted == 0) phase_lawson<true, true>(g, P, 0, stamp, lc, sc0);
-  else stamp = repair_step(g, P, stamp, q0);
+  else if (P.substeps > 0 || (sparse && P.V_it > kStarSparse) || !star_step(g, P, stamp, q0, sc0, lc))
+    stamp = repair_step(g, P, stamp, q0);
   flush_counters(P, lc);
   // No closing grid barrier: each block leaves when its own work is done and
   // the last one to leave publishes the launch.  The block barrier orders its
@@ -2263,7 +2901,7 @@ void free_mesh(mcl_mesh* m) {
   if (!m) return;
   void* ptrs[] = {m->pos[0], m->pos[1], m->ev, m->en, m->vhe, m->vfix, m->cand, m->win, m->qmark, m->efa, m->hard,
                   m->wl[0], m->wl[1], m->vl[0], m->vl[1], m->vmark, m->claim, m->vfree, m->vhint,
-                  m->vaux, m->vloc, m->vlocf, m->target, m->vprev, m->vl2, m->dstage, m->scratch, m->st,
+                  m->vaux, m->vloc, m->vlocf, m->target, m->star, m->cebase, m->vprev, m->vl2, m->dstage, m->scratch, m->st,
                   m->vcomp, m->vroot, m->cbase, m->table, m->smark, m->smove, m->fnew, m->act_dev,
                   m->bg_cell, m->bg_src, m->bg_perm, m->bg_pos, m->bg_count, m->bg_start, m->bg_cursor,
                   m->bg_tmp, m->bg_par, m->aos_tmp};
@@ -2339,6 +2977,7 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   A((void**)&m->vloc, 4 * V);
   A((void**)&m->vlocf, 4 * V);
   A((void**)&m->target, 8 * V);
+  A((void**)&m->star, 4 * star_ints(V));
   A((void**)&m->dstage, 8 * V);
   A((void**)&m->scratch, 64);
   A((void**)&m->st, sizeof(DevState));
@@ -2354,6 +2993,7 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   if (e == cudaSuccess) e = cudaMemset(m->vaux, 0xff, 4 * V);
   if (e == cudaSuccess) e = cudaMemset(m->vhint, 0xff, 4 * V);
   if (e == cudaSuccess) e = cudaMemset(m->vmark, 0, 4 * V);
+  if (e == cudaSuccess) e = cudaMemset(m->star + star_mark_at(V), 0, 4 * V);
   DevState s;
   std::memset(&s, 0, sizeof(s));
   s.epoch = 1;
@@ -2542,6 +3182,16 @@ static KParams make_params(mcl_mesh* m, int mode) {
   P.target = m->target;
   P.vprev = m->vprev;
   P.vl2 = m->vl2;
+  P.srow = m->star;
+  P.sext = m->star + (int64_t)kRow * m->V;
+  P.smark = reinterpret_cast<unsigned*>(m->star + star_mark_at(m->V));
+  P.sblk = m->star + star_sums_at(m->V);
+  P.sinbox = P.sblk + 4 * kStarBlocks;
+  P.srank = reinterpret_cast<unsigned long long*>(m->target);
+  P.sbase = m->vloc;
+  P.vcomp = m->vcomp;
+  P.cbase = m->cbase;
+  P.cebase = m->cebase;
   P.st = m->st;
   P.mode = mode;
   P.max_rounds = 1 << 16;

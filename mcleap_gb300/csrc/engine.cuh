@@ -69,6 +69,9 @@ struct DevState {
   int mark_ovf;            // the repair's appended marks did not fit, or were not all appended
   int movers_now;          // vertices this launch's move pass moved
   int movers_last;         // ... the last launch's (whether this move pass lists them)
+  int star_n[3];           // vertices whose stars disagree, per round (triple-buffered; bit 30: given up)
+  int star_ext;            // overflow rows taken by this launch
+  int star_made;           // stars made anew by this launch
   int sub_count[3];        // repair sub-steps: mover lists (2), vertices left for removal
   int sub_rev[3];          // movers sent back per sub-step pass (triple-buffered)
   unsigned int epoch;      // next unused stamp
@@ -135,6 +138,16 @@ struct KParams {
   float2* vprev;           // per vertex: position before the current repair sub-step
   int* vl2;                // 4 x V: repair sub-step lists (movers x2, sent back, left for removal);
                            // vprev and vl2 exist only after mcl_mesh_set_substeps(m, n > 0)
+  int* srow;               // star rows, kRow ints per vertex (star.cuh)
+  int* sext;               // overflow rows
+  unsigned* smark;         // per vertex: stamp of the last round that listed it
+  int* sinbox;             // kInbox ints per vertex: vertices to consider in the next round
+  int* sblk;               // per block: sums of the star check
+  unsigned long long* srank;  // per vertex: ranks of its entries in their owners' rows (shares `target`)
+  int* sbase;              // per vertex: own edges of the vertices before it (shares `vloc`)
+  const int* vcomp;        // batches: mesh of a vertex, first vertex and first edge of a mesh (NULL: plain)
+  const int* cbase;
+  const int* cebase;
   DevState* st;
   // move inputs
   const float2* disp;
@@ -350,6 +363,7 @@ struct mcl_mesh {
   float2* target;
   float2* vprev;
   int* vl2;
+  int* star;               // star rows, overflow rows, marks and block sums in one allocation
   float2* dstage;          // device staging buffer for host displacements
   // mcl_step_host_async: a second staging buffer, a copy stream, and events
   float2* dstage2;
@@ -377,6 +391,7 @@ struct mcl_mesh {
   int* vcomp;              // per vertex: component (NULL for a plain mesh)
   int* vroot;              // per vertex: half-edge 0 of its component (NULL for a plain mesh)
   int* cbase;              // per component: first vertex (NULL for a plain mesh)
+  int* cebase;             // per component: first edge (NULL for a plain mesh)
   // mcl_settle_moves
   unsigned long long* table;  // hash table of positions, stamped entries
   int64_t table_size;
