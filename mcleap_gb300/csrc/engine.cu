@@ -2979,9 +2979,11 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   A((void**)&m->target, 8 * V);
   A((void**)&m->star, 4 * star_ints(V));
   A((void**)&m->dstage, 8 * V);
-  A((void**)&m->scratch, 64);
+  A((void**)&m->scratch, kScratchBytes);
   A((void**)&m->st, sizeof(DevState));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&m->st_host, sizeof(DevState));
+  // the mirror of the device state, and behind it the counts that queries write
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&m->st_host, sizeof(DevState) + 64);
+  if (e == cudaSuccess) m->counts_host = reinterpret_cast<unsigned long long*>(m->st_host + 1);
   if (e != cudaSuccess) {
     free_mesh(m);
     return cuda_fail(e, "cudaMalloc(mesh)");
@@ -2993,6 +2995,7 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   if (e == cudaSuccess) e = cudaMemset(m->vaux, 0xff, 4 * V);
   if (e == cudaSuccess) e = cudaMemset(m->vhint, 0xff, 4 * V);
   if (e == cudaSuccess) e = cudaMemset(m->vmark, 0, 4 * V);
+  if (e == cudaSuccess) e = cudaMemset(m->scratch, 0, kScratchBytes);
   if (e == cudaSuccess) e = cudaMemset(m->star + star_mark_at(V), 0, 4 * V);
   DevState s;
   std::memset(&s, 0, sizeof(s));

@@ -371,7 +371,8 @@ struct mcl_mesh {
   cudaEvent_t ev_copied[2], ev_used[2];
   mcl_step_stats* stats_dev;  // [2] published counters of the pipelined steps
   int stage_idx;
-  unsigned long long* scratch;  // small device scratch for query counters
+  unsigned long long* scratch;  // small device scratch for query counters (kScratchBytes)
+  unsigned long long* counts_host;  // pinned, device-visible: counts of the last counted queries
   mcl::DevState* st;
   mcl::DevState* st_host;  // pinned mirror
   int coop_blocks;         // k_step grid
@@ -426,6 +427,7 @@ struct mcl_mesh {
 
 // Host-side helpers shared by the translation units of the library.
 namespace mcl {
+constexpr int kScratchBytes = 256;
 int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out);
 void free_mesh(mcl_mesh* m);
 int fail(int code, const std::string& msg);

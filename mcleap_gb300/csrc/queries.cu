@@ -60,44 +60,72 @@ __device__ __forceinline__ int mv_rot(const MeshView& M, int h) { return mv_next
 constexpr int kMaxDeg = 4096;
 
 // ---------------------------------------------------------------------------
-// Rings of up to kRegRing spokes are walked once and kept in shared memory,
-// then written starting at the spoke to the smallest neighbour; longer rings
-// walk twice.  (A register array indexed through unrolled compare-and-select
-// chains made the kernel instruction-bound: 71 % SM throughput at 53 us for
-// 1M vertices.)
-constexpr int kRegRing = 16;
-constexpr int kRingThreads = 256;
+// A count that the host waits for (truncated rings, overflowing lists): the
+// kernel adds to cell[0], and its last block writes the sum to pinned host memory
+// and leaves the cell at zero for the next call, so that a query is one launch and
+// one wait (a memset before and a copy after it cost a small query as much as the
+// kernel).  cell[1] counts the blocks that have finished.  A call that asks for no
+// count passes no cell.
+__device__ __forceinline__ void count_done(unsigned long long* cell, unsigned long long* host) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(cell + 1, 1ull) == gridDim.x - 1) {
+      __threadfence();
+      *host = atomicExch(cell, 0ull);
+      cell[1] = 0;
+    }
+  }
+}
 
-__global__ void __launch_bounds__(kRingThreads) k_one_ring(MeshView M, int layout, int max_ring, int* ring,
-                                                  unsigned long long* truncated) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M.V) return;
-  const int h0 = __ldg(M.vhe + i);
-  if (h0 < 0) return;
-  const int cap = max_ring - 1;
-  const size_t stride = layout == MCL_LAYOUT_COLUMN ? (size_t)M.V : 1;
-  int* row = layout == MCL_LAYOUT_COLUMN ? ring + i : ring + (size_t)i * max_ring;
-  // the first kRegRing neighbours in walk order, one column per thread
-  // (conflict-free), rotated to start at the smallest when written out
-  __shared__ int sring[kRegRing][kRingThreads];
-  int start = h0, best = 0x7fffffff, deg = 0, at = 0;
-  int h = h0;
+// One-ring, one thread per vertex.  What bounds it is the chain of dependent
+// record reads, so the ring is walked both ways at once: the record of a spoke links
+// to both its neighbours, and a ring of six closes after three links.  The record
+// of spoke k holds its own end and, as the apexes of its two faces, the ends of
+// spokes k - 1 and k + 1, so the ends are read at every other spoke.  Rings of up to
+// 15 spokes are kept in shared memory, then written starting at the smallest
+// neighbour; a row layout is written by four lanes per row, four words each (a thread
+// per row wrote seven words of 32 rows apart).  Longer rings and the rings
+// of the corners (next to the outside, which has no apex) are walked spoke by spoke.
+//
+// A corner's ring can have hundreds of spokes when points sit on the sides of their
+// box.  Its smallest neighbour is one of the two corners beside it (corners have
+// the smallest ids of their mesh, and in a Delaunay mesh with a point no corner
+// meets the one across), next to each other around the outside: its ring is written
+// from there at once, and no further than the row.
+//
+// GB300, before (both records of every spoke in turn, corners walked whole) -> now:
+// 1M points advected, column layout 50.9 -> 45 us (107 MB read); 500,000 points, row
+// layout 49.2 -> 36.0 us; the precision-stress set of 500,000 after random walks
+// (corners with long rings) 50.8 -> 24.0 us; 96 meshes of 1.4M points 83 -> 57 us.
+constexpr int kRegRing = 16;
+constexpr int kRingThreads = 128;
+
+__device__ __noinline__ void ring_walk(const MeshView M, int h0, int cap, size_t stride, int* row, bool corner_first,
+                                       unsigned long long* truncated) {
+  int start = h0, best = 0x7fffffff, deg = 0, h = h0;
+  if (corner_first) {
+    const int h1 = mv_rot(M, h0);
+    start = h = mv_origin(M, h0 ^ 1) < mv_origin(M, h1 ^ 1) ? h0 : h1;
+    do {
+      row[(size_t)(deg + 1) * stride] = mv_origin(M, h ^ 1);
+      h = mv_rot(M, h);
+      ++deg;
+    } while (h != start && deg < cap);
+    if (deg > 3 || h != start) {  // (a square with no point has its diagonal)
+      row[0] = deg;
+      if (truncated && h != start) atomicAdd(truncated, 1ull);
+      return;
+    }
+    h = start = h0;
+    deg = 0;
+  }
   do {
     const int w = mv_origin(M, h ^ 1);
-    if (w < best) { best = w; start = h; at = deg; }
-    if (deg < kRegRing) sring[deg][threadIdx.x] = w;
+    if (w < best) { best = w; start = h; }
     h = mv_rot(M, h);
     ++deg;
   } while (h != h0 && deg < kMaxDeg);
-  if (deg <= kRegRing && deg <= cap) {
-    int src = at;
-    for (int k = 0; k < deg; ++k) {
-      row[(size_t)(k + 1) * stride] = sring[src][threadIdx.x];
-      if (++src == deg) src = 0;
-    }
-    row[0] = deg;
-    return;
-  }
   const int cnt = deg < cap ? deg : cap;
   h = start;
   for (int k = 0; k < cnt; ++k) {
@@ -105,40 +133,158 @@ __global__ void __launch_bounds__(kRingThreads) k_one_ring(MeshView M, int layou
     h = mv_rot(M, h);
   }
   row[0] = cnt;
-  if (deg > cap) atomicAdd(truncated, 1ull);
+  if (truncated && deg > cap) atomicAdd(truncated, 1ull);
 }
 
+// Rows for the vertices verts[0 .. n) (NULL: all of them).  delaunay: the mesh is a
+// Delaunay triangulation; vfix marks the corners.
+template <bool kRow>
+__global__ void __launch_bounds__(kRingThreads) k_one_ring(MeshView M, const int* __restrict__ verts, int n,
+                                                           int max_ring, int* ring,
+                                                           const unsigned char* __restrict__ vfix, int delaunay,
+                                                           unsigned long long* truncated, unsigned long long* host) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int i = q < n ? (verts ? __ldg(verts + q) : q) : -1;
+  const int h0 = i >= 0 && i < M.V ? __ldg(M.vhe + i) : -1;
+  const int cap = max_ring - 1;
+  const size_t stride = kRow ? 1 : (size_t)n;
+  int* row = kRow ? ring + (size_t)q * max_ring : ring + q;
+  if (verts && q < n && h0 < 0) row[0] = 0;
+  // neighbour k of the walk (negative: the other way) in slot k mod kRegRing, one
+  // column per thread (conflict-free)
+  __shared__ int sring[kRegRing][kRingThreads];
+  int deg = 0, at = 0;
+  bool done = h0 < 0;
+  if (!done) {
+    int* col = &sring[0][threadIdx.x];
+    int best = 0x7fffffff;
+    bool plain = true;
+    auto keep = [&](int k, int w) {
+      plain = plain && w >= 0;
+      col[(k & (kRegRing - 1)) * kRingThreads] = w;
+      if (w < best) { best = w; at = k; }
+    };
+    const int4 n0 = __ldg(M.en + (h0 >> 1)), e0 = __ldg(M.ev + (h0 >> 1));
+    int a = (h0 & 1) ? n0.x : n0.z, b = ((h0 & 1) ? n0.w : n0.y) ^ 1;  // spokes 1 and -1
+    keep(0, (h0 & 1) ? e0.x : e0.y);
+    keep(1, (h0 & 1) ? e0.z : e0.w);
+    keep(-1, (h0 & 1) ? e0.w : e0.z);
+    for (int k = 1; plain && k < kRegRing / 2; ++k) {
+      // spokes k and -k; the records of the even ones hold the ends around them
+      if (k & 1) {
+        if (a == b) { deg = 2 * k; break; }
+      }
+      const int4 na = __ldg(M.en + (a >> 1)), nb = __ldg(M.en + (b >> 1));
+      if (!(k & 1)) {
+        const int4 ea = __ldg(M.ev + (a >> 1)), eb = __ldg(M.ev + (b >> 1));
+        keep(k, (a & 1) ? ea.x : ea.y);
+        if (a == b) { deg = 2 * k; break; }
+        keep(-k, (b & 1) ? eb.x : eb.y);
+        if (k + 1 < kRegRing / 2) {
+          keep(k + 1, (a & 1) ? ea.z : ea.w);
+          keep(-k - 1, (b & 1) ? eb.w : eb.z);
+        }
+      }
+      const int a1 = (a & 1) ? na.x : na.z;
+      if (a1 == b) { deg = 2 * k + 1; break; }
+      a = a1;
+      b = ((b & 1) ? nb.w : nb.y) ^ 1;
+      plain = plain && a >= 0 && b >= 0;
+    }
+    if (!plain || !deg || deg > cap) {
+      bool corners = false;
+      if (delaunay && vfix[i]) {
+        const int c = mv_origin(M, h0 ^ 1), d = mv_origin(M, mv_rot(M, h0) ^ 1);
+        corners = vfix[c] && vfix[d];
+      }
+      ring_walk(M, h0, cap, stride, row, corners, truncated);
+      done = true;
+    }
+  }
+  if (kRow) {
+    __syncwarp();
+    // eight rows a turn, four lanes each, four words a lane (one store where the row
+    // lies on 16 bytes and all four are written: slots past the ring stay as they are)
+    const int j = 4 * (lane & 3), first = q - lane;
+    const bool vec = ((max_ring & 3) | (int)((size_t)ring & 15)) == 0;
+    for (int r = 0; r < 32; r += 8) {
+      const int src = r + (lane >> 2);
+      const int d = __shfl_sync(0xffffffffu, deg, src), a = __shfl_sync(0xffffffffu, at, src);
+      const bool skip = __shfl_sync(0xffffffffu, (int)done, src) != 0;
+      if (skip || j > d) continue;
+      int x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        // entry j + k - 1 from the smallest: the ring index in -(d - 1) / 2 .. d / 2
+        int o = a + j + k - 1;
+        if (o > d / 2) o -= d;
+        x[k] = j + k == 0 ? d : sring[o & (kRegRing - 1)][(threadIdx.x & ~31) + src];
+      }
+      int* to = ring + (size_t)(first + src) * max_ring + j;
+      if (vec && j + 3 <= d) {
+        *reinterpret_cast<int4*>(to) = make_int4(x[0], x[1], x[2], x[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (j + k <= d) to[k] = x[k];
+      }
+    }
+  } else if (!done) {
+    int o = at;
+    for (int k = 0; k < deg; ++k) {
+      row[(size_t)(k + 1) * stride] = sring[o & (kRegRing - 1)][threadIdx.x];
+      if (++o > deg / 2) o -= deg;
+    }
+    row[0] = deg;
+  }
+  if (host) count_done(truncated, host);
+}
+
+// Nearest entry of each ring row.  kVec: rows are read four words at a time (row
+// layout, rows on 16 bytes: two loads for the usual ring instead of eight, each a
+// tag lookup per lane; 500,000 rows 22.1 -> 14.4 us).
+template <bool kVec>
 __global__ void k_closest(const float2* pos, int V, int layout, int max_ring, const int* ring, int* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
-  const int cnt = layout == MCL_LAYOUT_COLUMN ? ring[i] : ring[(size_t)i * max_ring];
   const float2 p = pos[i];
   int best = -1;
   float bd = 0.f;
-  for (int k = 0; k < cnt; ++k) {
-    const int j = layout == MCL_LAYOUT_COLUMN ? ring[(size_t)(k + 1) * V + i] : ring[(size_t)i * max_ring + k + 1];
+  auto look = [&](int j) {
     const float d = sqdist(p, pos[j]);
     if (best < 0 || d < bd || (d == bd && j < best)) { best = j; bd = d; }
+  };
+  if (kVec) {
+    const int4* row = reinterpret_cast<const int4*>(ring + (size_t)i * max_ring);
+    const int4 a = row[0];
+    const int cnt = a.x;
+    if (cnt > 0) look(a.y);
+    if (cnt > 1) look(a.z);
+    if (cnt > 2) look(a.w);
+    for (int k = 3; k < cnt; k += 4) {
+      const int4 b = row[(k + 1) >> 2];
+      look(b.x);
+      if (cnt > k + 1) look(b.y);
+      if (cnt > k + 2) look(b.z);
+      if (cnt > k + 3) look(b.w);
+    }
+  } else {
+    const int cnt = layout == MCL_LAYOUT_COLUMN ? ring[i] : ring[(size_t)i * max_ring];
+    for (int k = 0; k < cnt; ++k)
+      look(layout == MCL_LAYOUT_COLUMN ? ring[(size_t)(k + 1) * V + i] : ring[(size_t)i * max_ring + k + 1]);
   }
   out[i] = best;
 }
 
-// Mesh FRNN: depth-first search over the mesh from i through vertices within r
-// (the reference's getFRNN, include/Host_Triangulation.h:525-560 and
-// include/kernels.cuh:169-219).  The found set is kept in a thread-local list,
-// then written sorted ascending.
+// Mesh FRNN: search over the mesh from i through vertices within r (the
+// reference's getFRNN, include/Host_Triangulation.h:525-560 and
+// include/kernels.cuh:169-219); the found set is written sorted ascending.
 constexpr int kFrnnLocal = 256;
 
-// With rcomp != nullptr the radius of vertex i is rcomp[vcomp[i]] (one radius
-// per mesh of a batch; a plain mesh has vcomp == nullptr and one radius).
-__global__ void k_mesh_frnn(MeshView M, float r2, int layout, int max_frnn, int* out, unsigned long long* overflow,
-                            const float* rcomp, const int* vcomp) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M.V) return;
-  if (rcomp) {
-    const float rc = rcomp[vcomp ? vcomp[i] : 0];
-    r2 = __fmul_rn(rc, rc);
-  }
+// One thread's search, depth first, for sets that a warp's lists do not hold:
+// up to kFrnnLocal vertices, in a thread-local list.  Returns the count written.
+__device__ __noinline__ void frnn_serial(const MeshView M, int i, float r2, int cap, size_t stride, int* row,
+                                         unsigned long long* overflow) {
   int found[kFrnnLocal];
   int nf = 0;
   int top = 0;  // stack = found[top..nf): vertices whose rings are still to scan
@@ -167,22 +313,140 @@ __global__ void k_mesh_frnn(MeshView M, float r2, int layout, int max_frnn, int*
     if (top >= nf) break;
     cur = found[top++];
   }
-  // insertion sort
   for (int a = 1; a < nf; ++a) {
     const int x = found[a];
     int b = a - 1;
     while (b >= 0 && found[b] > x) { found[b + 1] = found[b]; --b; }
     found[b + 1] = x;
   }
-  const int cap = max_frnn - 1;
   const int cnt = nf < cap ? nf : cap;
-  for (int k = 0; k < cnt; ++k) {
-    if (layout == MCL_LAYOUT_COLUMN) out[(size_t)(k + 1) * M.V + i] = found[k];
-    else out[(size_t)i * max_frnn + k + 1] = found[k];
+  for (int k = 0; k < cnt; ++k) row[(size_t)(k + 1) * stride] = found[k];
+  row[0] = cnt;
+  if (overflow && (over || nf > cap)) atomicAdd(overflow, 1ull);
+}
+
+// A warp's search, breadth first: two lanes walk the ring of one vertex of the
+// frontier from its first spoke, one each way, until they meet; a lane's neighbour
+// within r joins through a hash set in shared memory.  The search is a chain of
+// dependent loads, so the time is the number of steps one after another: about
+// four a level for a ring of six, three or four levels for r = 2 x spacing, where a
+// thread alone takes a step for each of some eighty spokes and looks each up in its
+// own list in local memory.  60,000 queries, r = 2 x spacing, GB300: 567 us by
+// threads, 168 us by warps.
+constexpr int kFrnnWarps = 4;
+constexpr int kFrnnFound = 64;
+constexpr int kFrnnHash = 128;
+
+__device__ __forceinline__ int mv_prev(const MeshView& M, int h) {
+  return __ldg(reinterpret_cast<const int*>(M.en) + 4 * (h >> 1) + 2 * (h & 1) + 1);
+}
+
+__device__ __forceinline__ bool warp_search(const MeshView& M, int i, float r2, int* found, int* hash, int* count) {
+  const int lane = threadIdx.x & 31, way = lane & 1;
+  const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+  for (int k = 0; k < kFrnnHash / 32; ++k) hash[32 * k + lane] = -1;
+  __syncwarp();
+  const float2 pi = M.pos[i];
+  int nf = 0, lo = -1;  // the frontier: i, then found[lo .. hi)
+  while (lo < nf) {
+    const int hi = lo < 0 ? 0 : nf;
+    for (int c = lo; c < hi; c += 16) {
+      const int j = c + (lane >> 1);
+      const int u = lo < 0 ? (j == lo ? i : -1) : (j < hi ? found[j] : -1);
+      const int h0 = u >= 0 ? __ldg(M.vhe + u) : -1;
+      bool on = h0 >= 0;
+      int cur = h0;
+      if (on && way) {
+        cur = mv_prev(M, h0) ^ 1;
+        on = cur != h0;  // a ring of one spoke is the other lane's
+      }
+      bool last = !__shfl_xor_sync(0xffffffffu, (int)on, 1);
+      for (int step = 0; step < kMaxDeg && __any_sync(0xffffffffu, on); ++step) {
+        int w = -1, nxt = -1;
+        if (on) {
+          w = mv_origin(M, cur ^ 1);
+          nxt = way ? mv_prev(M, cur) ^ 1 : mv_rot(M, cur);
+        }
+        bool fresh = false;
+        if (on && w != i && w >= 0 && sqdist(pi, M.pos[w]) <= r2) {
+          unsigned k = ((unsigned)w * 2654435761u) >> 25;
+          for (;;) {
+            const int old = atomicCAS(hash + k, -1, w);
+            fresh = old == -1;
+            if (fresh || old == w) break;
+            k = (k + 1) & (kFrnnHash - 1);
+          }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, fresh);
+        if (fresh) {
+          const int at = nf + __popc(m & lt);
+          if (at < kFrnnFound) found[at] = w;
+        }
+        nf += __popc(m);
+        if (nf > kFrnnFound) return false;
+        const int ocur = __shfl_xor_sync(0xffffffffu, cur, 1), onxt = __shfl_xor_sync(0xffffffffu, nxt, 1);
+        if (on) {
+          if (last || nxt == ocur || nxt < 0) on = false;  // met, or the one between has been taken
+          else if (nxt == onxt) {                          // one between: this way takes it
+            last = true;
+            if (way) on = false;
+          }
+          cur = nxt;
+        }
+      }
+      __syncwarp();
+    }
+    lo = hi;
   }
-  if (layout == MCL_LAYOUT_COLUMN) out[i] = cnt;
-  else out[(size_t)i * max_frnn] = cnt;
-  if (over || nf > cap) atomicAdd(overflow, 1ull);
+  *count = nf;
+  return true;
+}
+
+// Rows for the vertices verts[0 .. n) (NULL: all of them), a warp each.  With
+// rcomp the radius of vertex i is rcomp[vcomp[i]] (one radius per mesh of a batch; a
+// plain mesh has vcomp == nullptr and one radius).
+__global__ void __launch_bounds__(32 * kFrnnWarps) k_mesh_frnn(MeshView M, const int* verts, int n, float r2,
+                                                               int layout, int max_frnn, int* out,
+                                                               unsigned long long* overflow,
+                                                               unsigned long long* host, const float* rcomp,
+                                                               const int* vcomp) {
+  __shared__ int found_s[kFrnnWarps][kFrnnFound];
+  __shared__ int hash_s[kFrnnWarps][kFrnnHash];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q = blockIdx.x * kFrnnWarps + warp;
+  if (q < n) {
+    const int i = verts ? __ldg(verts + q) : q;
+    const int cap = max_frnn - 1;
+    int* row = layout == MCL_LAYOUT_COLUMN ? out + q : out + (size_t)q * max_frnn;
+    const size_t stride = layout == MCL_LAYOUT_COLUMN ? (size_t)n : 1;
+    if (i < 0 || i >= M.V || __ldg(M.vhe + i) < 0) {
+      if (lane == 0) row[0] = 0;
+    } else {
+      if (rcomp) {
+        const float rc = rcomp[vcomp ? vcomp[i] : 0];
+        r2 = __fmul_rn(rc, rc);
+      }
+      int* found = found_s[warp];
+      int nf = 0;
+      if (warp_search(M, i, r2, found, hash_s[warp], &nf)) {
+        __syncwarp();
+        for (int k = lane; k < nf; k += 32) {
+          const int x = found[k];
+          int rank = 0;
+          for (int j = 0; j < nf; ++j) rank += found[j] < x ? 1 : 0;
+          if (rank < cap) row[(size_t)(rank + 1) * stride] = x;
+        }
+        if (lane == 0) {
+          row[0] = nf < cap ? nf : cap;
+          if (overflow && nf > cap) atomicAdd(overflow, 1ull);
+        }
+      } else if (lane == 0) {
+        frnn_serial(M, i, r2, cap, stride, row, overflow);
+      }
+    }
+  }
+  if (host) count_done(overflow, host);
 }
 
 // Diffusion-limited aggregation contact (the reference's check_if_close_diffusion,
@@ -237,90 +501,6 @@ __global__ void k_dla_commit(ActV A, unsigned char* frozen, const unsigned char*
   if (ii >= A.V_it) return;
   const int i = A.at(ii);
   frozen[i] = fnew[i];
-}
-
-// Mesh FRNN / one-ring for a list of query vertices: row q is verts[q].
-__global__ void k_mesh_frnn_list(MeshView M, const float* rcomp, const int* vcomp, const int* verts, int n, int layout,
-                                 int max_frnn, int* out, unsigned long long* overflow) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int i = verts[q];
-  const int cap = max_frnn - 1;
-  int* row = layout == MCL_LAYOUT_COLUMN ? out + q : out + (size_t)q * max_frnn;
-  const size_t stride = layout == MCL_LAYOUT_COLUMN ? (size_t)n : 1;
-  if (i < 0 || i >= M.V || __ldg(M.vhe + i) < 0) {
-    row[0] = 0;
-    return;
-  }
-  const float rc = rcomp[vcomp ? vcomp[i] : 0];
-  const float r2 = __fmul_rn(rc, rc);
-  int found[kFrnnLocal];
-  int nf = 0, top = 0;
-  bool over = false;
-  const float2 pi = M.pos[i];
-  int cur = i;
-  for (int guard = 0; guard < (1 << 20); ++guard) {
-    const int h0 = __ldg(M.vhe + cur);
-    if (h0 >= 0) {
-      int h = h0, deg = 0;
-      do {
-        const int w = mv_origin(M, h ^ 1);
-        if (w != i) {
-          bool seen = false;
-          for (int k = 0; k < nf; ++k)
-            if (found[k] == w) { seen = true; break; }
-          if (!seen && sqdist(pi, M.pos[w]) <= r2) {
-            if (nf < kFrnnLocal) found[nf++] = w;
-            else over = true;
-          }
-        }
-        h = mv_rot(M, h);
-        ++deg;
-      } while (h != h0 && deg < kMaxDeg);
-    }
-    if (top >= nf) break;
-    cur = found[top++];
-  }
-  for (int a = 1; a < nf; ++a) {
-    const int x = found[a];
-    int b = a - 1;
-    while (b >= 0 && found[b] > x) { found[b + 1] = found[b]; --b; }
-    found[b + 1] = x;
-  }
-  const int cnt = nf < cap ? nf : cap;
-  for (int k = 0; k < cnt; ++k) row[(size_t)(k + 1) * stride] = found[k];
-  row[0] = cnt;
-  if (over || nf > cap) atomicAdd(overflow, 1ull);
-}
-
-__global__ void k_one_ring_list(MeshView M, const int* verts, int n, int layout, int max_ring, int* out,
-                                unsigned long long* truncated) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int i = verts[q];
-  int* row = layout == MCL_LAYOUT_COLUMN ? out + q : out + (size_t)q * max_ring;
-  const size_t stride = layout == MCL_LAYOUT_COLUMN ? (size_t)n : 1;
-  const int h0 = (i >= 0 && i < M.V) ? __ldg(M.vhe + i) : -1;
-  if (h0 < 0) {
-    row[0] = 0;
-    return;
-  }
-  int start = h0, best = 0x7fffffff, deg = 0, h = h0;
-  do {
-    const int w = mv_origin(M, h ^ 1);
-    if (w < best) { best = w; start = h; }
-    h = mv_rot(M, h);
-    ++deg;
-  } while (h != h0 && deg < kMaxDeg);
-  const int cap = max_ring - 1;
-  const int cnt = deg < cap ? deg : cap;
-  h = start;
-  for (int k = 0; k < cnt; ++k) {
-    row[(size_t)(k + 1) * stride] = mv_origin(M, h ^ 1);
-    h = mv_rot(M, h);
-  }
-  row[0] = cnt;
-  if (deg > cap) atomicAdd(truncated, 1ull);
 }
 
 }  // namespace
@@ -715,6 +895,57 @@ __global__ void k_debug_pred(int kind, const float* pts, const int* ids, int64_t
 
 }  // namespace
 
+namespace {
+
+// Counted queries: a cell pair per kind in the mesh's device scratch, a slot per
+// kind in its pinned host memory (count_done).
+enum { kCellRing = 8, kCellFrnn = 10, kHostRing = 0, kHostFrnn = 1 };
+
+MeshView mesh_view(const mcl_mesh* m) {
+  return MeshView{m->ev, m->en, m->vhe, m->pos[m->cur], (int)m->V, (int)m->E};
+}
+
+int wait_count(unsigned long long* host, cudaStream_t s, int64_t* out) {
+  if (!out) return MCL_OK;
+  QCK(cudaStreamSynchronize(s));
+  *out = (int64_t) * (volatile unsigned long long*)host;
+  return MCL_OK;
+}
+
+int launch_one_ring(mcl_mesh* m, const int* verts, int64_t n, int layout, int max_ring, int* out, cudaStream_t s,
+                    int64_t* truncated) {
+  if (n == 0) {
+    if (truncated) QCK(cudaStreamSynchronize(s));
+    if (truncated) *truncated = 0;
+    return MCL_OK;
+  }
+  const unsigned blocks = (unsigned)((n + kRingThreads - 1) / kRingThreads);
+  const int delaunay = m->delaunay && m->valid_cur ? 1 : 0;
+  unsigned long long* host = truncated ? m->counts_host + kHostRing : nullptr;
+  auto kernel = layout == MCL_LAYOUT_COLUMN ? k_one_ring<false> : k_one_ring<true>;
+  kernel<<<blocks, kRingThreads, 0, s>>>(mesh_view(m), verts, (int)n, max_ring, out, m->vfix, delaunay,
+                                         host ? m->scratch + kCellRing : nullptr, host);
+  QCK(cudaGetLastError());
+  return wait_count(host, s, truncated);
+}
+
+int launch_mesh_frnn(mcl_mesh* m, const int* verts, int64_t n, float r2, const float* rcomp, int layout, int max_frnn,
+                     int* out, cudaStream_t s, int64_t* overflow) {
+  if (n == 0) {
+    if (overflow) QCK(cudaStreamSynchronize(s));
+    if (overflow) *overflow = 0;
+    return MCL_OK;
+  }
+  unsigned long long* host = overflow ? m->counts_host + kHostFrnn : nullptr;
+  k_mesh_frnn<<<(unsigned)((n + kFrnnWarps - 1) / kFrnnWarps), 32 * kFrnnWarps, 0, s>>>(
+      mesh_view(m), verts, (int)n, r2, layout, max_frnn, out, host ? m->scratch + kCellFrnn : nullptr, host, rcomp,
+      rcomp ? m->vcomp : nullptr);
+  QCK(cudaGetLastError());
+  return wait_count(host, s, overflow);
+}
+
+}  // namespace
+
 extern "C" {
 
 int mcl_debug_predicates_host(int kind, const float* pts, const int32_t* ids, int64_t n, int32_t* sign,
@@ -741,65 +972,29 @@ int mcl_debug_predicates_device(int kind, const float* pts, const int32_t* ids, 
 int mcl_one_ring(mcl_mesh* m, int layout, int max_ring, int32_t* ring, void* stream, int64_t* truncated) {
   if (!m || !ring || max_ring < 2 || (layout != MCL_LAYOUT_COLUMN && layout != MCL_LAYOUT_ROW))
     return qfail(MCL_ERR_INVALID_ARGUMENT, "bad args");
-  cudaStream_t s = (cudaStream_t)stream;
-  unsigned long long* cnt = m->scratch;
-  MeshView M{m->ev, m->en, m->vhe, m->pos[m->cur], (int)m->V, (int)m->E};
-  QCK(cudaMemsetAsync(cnt, 0, 8, s));
-  k_one_ring<<<(unsigned)((m->V + kRingThreads - 1) / kRingThreads), kRingThreads, 0, s>>>(M, layout, max_ring, ring,
-                                                                                          cnt);
-  QCK(cudaGetLastError());
-  if (truncated) {
-    unsigned long long t = 0;
-    QCK(cudaMemcpyAsync(&t, cnt, 8, cudaMemcpyDeviceToHost, s));
-    QCK(cudaStreamSynchronize(s));
-    *truncated = (int64_t)t;
-  }
-  return MCL_OK;
+  return launch_one_ring(m, nullptr, m->V, layout, max_ring, ring, (cudaStream_t)stream, truncated);
 }
 
 int mcl_closest_neighbors(mcl_mesh* m, int layout, int max_ring, const int32_t* ring, int32_t* out, void* stream) {
   if (!m || !ring || !out || max_ring < 2) return qfail(MCL_ERR_INVALID_ARGUMENT, "bad args");
-  k_closest<<<(unsigned)((m->V + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m->pos[m->cur], (int)m->V, layout,
-                                                                              max_ring, ring, out);
+  const bool vec = layout != MCL_LAYOUT_COLUMN && max_ring % 4 == 0 && ((uintptr_t)ring & 15) == 0;
+  auto kernel = vec ? k_closest<true> : k_closest<false>;
+  kernel<<<(unsigned)((m->V + 255) / 256), 256, 0, (cudaStream_t)stream>>>(m->pos[m->cur], (int)m->V, layout, max_ring,
+                                                                          ring, out);
   QCK(cudaGetLastError());
   return MCL_OK;
 }
 
 int mcl_mesh_frnn(mcl_mesh* m, float r, int layout, int max_frnn, int32_t* out, void* stream, int64_t* overflow) {
   if (!m || !out || max_frnn < 2 || !(r >= 0.f)) return qfail(MCL_ERR_INVALID_ARGUMENT, "bad args");
-  cudaStream_t s = (cudaStream_t)stream;
-  unsigned long long* cnt = m->scratch;
-  MeshView M{m->ev, m->en, m->vhe, m->pos[m->cur], (int)m->V, (int)m->E};
-  QCK(cudaMemsetAsync(cnt, 0, 8, s));
-  k_mesh_frnn<<<(unsigned)((m->V + 127) / 128), 128, 0, s>>>(M, r * r, layout, max_frnn, out, cnt, nullptr,
-                                                               nullptr);
-  QCK(cudaGetLastError());
-  if (overflow) {
-    unsigned long long t = 0;
-    QCK(cudaMemcpyAsync(&t, cnt, 8, cudaMemcpyDeviceToHost, s));
-    QCK(cudaStreamSynchronize(s));
-    *overflow = (int64_t)t;
-  }
-  return MCL_OK;
+  return launch_mesh_frnn(m, nullptr, m->V, r * r, nullptr, layout, max_frnn, out, (cudaStream_t)stream, overflow);
 }
 
 int mcl_batch_frnn(mcl_mesh* m, const float* r_dev, int layout, int max_frnn, int32_t* out, void* stream,
                    int64_t* overflow) {
   if (!m || !r_dev || !out || max_frnn < 2 || (layout != MCL_LAYOUT_COLUMN && layout != MCL_LAYOUT_ROW))
     return qfail(MCL_ERR_INVALID_ARGUMENT, "bad args");
-  cudaStream_t s = (cudaStream_t)stream;
-  unsigned long long* cnt = m->scratch;
-  MeshView M{m->ev, m->en, m->vhe, m->pos[m->cur], (int)m->V, (int)m->E};
-  QCK(cudaMemsetAsync(cnt, 0, 8, s));
-  k_mesh_frnn<<<(unsigned)((m->V + 127) / 128), 128, 0, s>>>(M, 0.f, layout, max_frnn, out, cnt, r_dev, m->vcomp);
-  QCK(cudaGetLastError());
-  if (overflow) {
-    unsigned long long t = 0;
-    QCK(cudaMemcpyAsync(&t, cnt, 8, cudaMemcpyDeviceToHost, s));
-    QCK(cudaStreamSynchronize(s));
-    *overflow = (int64_t)t;
-  }
-  return MCL_OK;
+  return launch_mesh_frnn(m, nullptr, m->V, 0.f, r_dev, layout, max_frnn, out, (cudaStream_t)stream, overflow);
 }
 
 int mcl_batch_frnn_list(mcl_mesh* m, const float* r_dev, const int32_t* verts_dev, int64_t n, int layout,
@@ -807,22 +1002,7 @@ int mcl_batch_frnn_list(mcl_mesh* m, const float* r_dev, const int32_t* verts_de
   if (!m || !r_dev || (n > 0 && (!verts_dev || !out_dev)) || n < 0 || max_frnn < 2 ||
       (layout != MCL_LAYOUT_COLUMN && layout != MCL_LAYOUT_ROW))
     return qfail(MCL_ERR_INVALID_ARGUMENT, "bad args");
-  cudaStream_t s = (cudaStream_t)stream;
-  unsigned long long* cnt = m->scratch + 2;
-  QCK(cudaMemsetAsync(cnt, 0, 8, s));
-  if (n > 0) {
-    MeshView M{m->ev, m->en, m->vhe, m->pos[m->cur], (int)m->V, (int)m->E};
-    k_mesh_frnn_list<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(M, r_dev, m->vcomp, verts_dev, (int)n, layout,
-                                                                 max_frnn, out_dev, cnt);
-    QCK(cudaGetLastError());
-  }
-  if (overflow) {
-    unsigned long long t = 0;
-    QCK(cudaMemcpyAsync(&t, cnt, 8, cudaMemcpyDeviceToHost, s));
-    QCK(cudaStreamSynchronize(s));
-    *overflow = (int64_t)t;
-  }
-  return MCL_OK;
+  return launch_mesh_frnn(m, verts_dev, n, 0.f, r_dev, layout, max_frnn, out_dev, (cudaStream_t)stream, overflow);
 }
 
 int mcl_one_ring_list(mcl_mesh* m, const int32_t* verts_dev, int64_t n, int layout, int max_ring, int32_t* out_dev,
@@ -830,21 +1010,7 @@ int mcl_one_ring_list(mcl_mesh* m, const int32_t* verts_dev, int64_t n, int layo
   if (!m || (n > 0 && (!verts_dev || !out_dev)) || n < 0 || max_ring < 2 ||
       (layout != MCL_LAYOUT_COLUMN && layout != MCL_LAYOUT_ROW))
     return qfail(MCL_ERR_INVALID_ARGUMENT, "bad args");
-  cudaStream_t s = (cudaStream_t)stream;
-  unsigned long long* cnt = m->scratch + 3;
-  QCK(cudaMemsetAsync(cnt, 0, 8, s));
-  if (n > 0) {
-    MeshView M{m->ev, m->en, m->vhe, m->pos[m->cur], (int)m->V, (int)m->E};
-    k_one_ring_list<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(M, verts_dev, (int)n, layout, max_ring, out_dev, cnt);
-    QCK(cudaGetLastError());
-  }
-  if (truncated) {
-    unsigned long long t = 0;
-    QCK(cudaMemcpyAsync(&t, cnt, 8, cudaMemcpyDeviceToHost, s));
-    QCK(cudaStreamSynchronize(s));
-    *truncated = (int64_t)t;
-  }
-  return MCL_OK;
+  return launch_one_ring(m, verts_dev, n, layout, max_ring, out_dev, (cudaStream_t)stream, truncated);
 }
 
 int mcl_dla_freeze(mcl_mesh* m, const float* r_dev, uint8_t* frozen, void* stream, int64_t* newly_frozen) {
