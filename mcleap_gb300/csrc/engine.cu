@@ -323,8 +323,9 @@ constexpr int kEvStages = 2;
 // a face turned over): kWarpBuf entries per warp each.  One block of shared
 // memory, which the star phases use whole for their candidate lists.
 constexpr int kEvSlots = kEvStages * kClassifyUnroll * kThreads;
-constexpr int kPool = kEvSlots + 2 * (kThreads / 32) * kWarpBuf / 4;
-constexpr int kStarSlots = kPool / kThreads;  // candidates per thread in the pool
+constexpr int kStarSlots = 15;  // candidates per thread in the pool
+constexpr int kPool = kStarSlots * 12 * kThreads / 16;
+static_assert(kPool >= kEvSlots + 2 * (kThreads / 32) * kWarpBuf / 4, "the staging slots and buffers fit");
 __shared__ int4 s_pool[kPool];
 __device__ __forceinline__ int4* ev_slot(int stage, int j) {
   return s_pool + (stage * kClassifyUnroll + j) * kThreads + threadIdx.x;
@@ -2226,17 +2227,23 @@ __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, 
 // Untangling by stars (star.cuh) inside the step's launch.
 
 // A vertex's candidates in this thread's slots of the shared pool (idle after
-// the classification).
+// the classification): a place and an id each, twelve bytes.
 struct SharedCand {
   MCL_HD int cap() const { return kStarSlots; }
-  __device__ __forceinline__ static float4* at(int i) {
-    return reinterpret_cast<float4*>(s_pool) + i * kThreads + threadIdx.x;
+  __device__ __forceinline__ static float2* at(int i) {
+    return reinterpret_cast<float2*>(s_pool) + i * kThreads + threadIdx.x;
+  }
+  __device__ __forceinline__ static int* who(int i) {
+    return reinterpret_cast<int*>(s_pool) + (2 * kStarSlots + i) * kThreads + threadIdx.x;
   }
   __device__ __forceinline__ Cand get(int i) const {
-    const float4 q = *at(i);
-    return Cand{q.x, q.y, q.z, __float_as_int(q.w)};
+    const float2 q = *at(i);
+    return Cand{q.x, q.y, *who(i)};
   }
-  __device__ __forceinline__ void set(int i, Cand c) { *at(i) = make_float4(c.x, c.y, c.key, __int_as_float(c.id)); }
+  __device__ __forceinline__ void set(int i, Cand c) {
+    *at(i) = make_float2(c.x, c.y);
+    *who(i) = c.id;
+  }
 };
 
 // The same for any number of candidates, in local memory: the vertices that
@@ -2266,10 +2273,14 @@ __device__ __forceinline__ bool warp_star(const KParams& P, int v, MeshBase mb, 
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const float2 pv = P.pos[v];
-  float4* slot = reinterpret_cast<float4*>(s_pool) + (threadIdx.x & ~31);
+  // the warp's slots: the first two records' places in its own threads' columns
+  // (SharedCand), 256 bytes each, so that no other warp's candidates are touched
+  auto slot = [&](int i) {
+    return reinterpret_cast<float4*>(SharedCand::at(i >> 4) - threadIdx.x + (threadIdx.x & ~31)) + (i & 15);
+  };
   auto at = [&](int i) {
-    const float4 q = slot[i];
-    return Cand{q.x, q.y, q.z, __float_as_int(q.w)};
+    const float4 q = *slot(i);
+    return Cand{q.x, q.y, __float_as_int(q.w)};
   };
   unsigned alive = 0;
   int p = 0, s = 0;
@@ -2296,13 +2307,13 @@ __device__ __forceinline__ bool warp_star(const KParams& P, int v, MeshBase mb, 
       live = __ballot_sync(kFull, valid);
       if (valid) valid = __ffs(__match_any_sync(live, x)) - 1 == lane;
     }
-    c = valid ? star_cand(pv, x, P.pos[x], 0.f) : Cand{0.f, 0.f, 0.f, -1};
-    if (__any_sync(kFull, valid && !(c.key >= 0.f))) return false;
+    c = valid ? star_cand(pv, x, P.pos[x]) : Cand{0.f, 0.f, -1};
+    float key = valid ? star_key(c, 0.f) : 0.f;
+    if (__any_sync(kFull, !(key >= 0.f))) return false;
     live = __ballot_sync(kFull, valid);
     if (__popc(live) < 3) continue;
-    const float from = __shfl_sync(kFull, c.key, __ffs(live) - 1);
-    c.key -= from;
-    if (c.key < 0.f) c.key += 4.f;
+    key -= __shfl_sync(kFull, key, __ffs(live) - 1);
+    if (key < 0.f) key += 4.f;
     // place in the angular order; of two on one ray the farther leaves
     int rank = 0;
     for (;;) {
@@ -2310,9 +2321,9 @@ __device__ __forceinline__ bool warp_star(const KParams& P, int v, MeshBase mb, 
       bool out = false, same = false;
       for (unsigned m = live; m; m &= m - 1) {
         const int j = __ffs(m) - 1;
-        const float kj = __shfl_sync(kFull, c.key, j);
-        bool before = kj < c.key;
-        const bool near = valid && j != lane && fabsf(kj - c.key) < kStarSameKey;
+        const float kj = __shfl_sync(kFull, key, j);
+        bool before = kj < key;
+        const bool near = valid && j != lane && fabsf(kj - key) < kStarSameKey;
         if (__any_sync(kFull, near)) {
           Cand u;
           u.x = __shfl_sync(kFull, c.x, j);
@@ -2343,7 +2354,7 @@ __device__ __forceinline__ bool warp_star(const KParams& P, int v, MeshBase mb, 
     }
     const int n = __popc(live);
     __syncwarp();
-    if (valid) slot[rank] = make_float4(c.x, c.y, c.key, __int_as_float(c.id));
+    if (valid) *slot(rank) = make_float4(c.x, c.y, 0.f, __int_as_float(c.id));
     __syncwarp();
     alive = n == 32 ? kFull : (1u << n) - 1u;
     c = at(lane < n ? lane : 0);
@@ -2578,6 +2589,20 @@ __device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, 
 // path, whose cost goes with the movers; the stars' goes with the mesh.
 constexpr int kStarSparse = 200000;
 
+// The vertices of the block's run marked with cs, in order, onto a list.
+__device__ __forceinline__ void star_marked(const KParams& P, unsigned cs, int i0, int i1, int* list, int* count) {
+  const int lane = threadIdx.x & 31;
+  WarpBuf wb{warp_buf(0), 0};
+  for (int base = i0 + (int)(threadIdx.x & ~31); base < i1; base += kThreads) {
+    const int i = base + lane;
+    const int v = i < i1 ? vert_at(P, i) : 0;
+    const int mine[1] = {v};
+    const int k = i < i1 && (unsigned)ld_i(reinterpret_cast<const int*>(P.smark) + v) == cs ? 1 : 0;
+    if (__any_sync(kFull, k)) wb_push(wb, mine, k, list, count, P.V, P.st);
+  }
+  wb_flush(wb, list, count, P.V, P.st);
+}
+
 // Vertices (or list entries) per warp of the launch up to which a warp takes one
 // vertex at a time; above it a thread does.
 constexpr int kWarpStars = 8;
@@ -2707,76 +2732,77 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
       g.sync();  // the sums have been read
       continue;
     }
-    // the marked vertices, listed in order
-    {
-      WarpBuf wb{warp_buf(0), 0};
-      for (int base = i0 + (int)(threadIdx.x & ~31); base < i1; base += kThreads) {
-        const int i = base + lane;
-        const int v = i < i1 ? vert_at(P, i) : 0;
-        const int mine[1] = {v};
-        const int k = i < i1 && (unsigned)ld_i(reinterpret_cast<const int*>(P.smark) + v) == cs ? 1 : 0;
-        if (__any_sync(kFull, k)) wb_push(wb, mine, k, lists[slot & 1], cnt + slot % 3, P.V, P.st);
-      }
-      wb_flush(wb, lists[slot & 1], cnt + slot % 3, P.V, P.st);
-    }
+    star_marked(P, cs, i0, i1, lists[slot & 1], cnt + slot % 3);
     g.sync();
     int n = ld_i(cnt + slot % 3);
-    if (n > kWarpStars * nwarps) {
-      // many stars disagree: a thread makes one, then everything is checked
-      if (++rounds > kStarRounds) return false;
-      fine = true;
-      for (int base = gwarp * 32; base < n; base += stride) {
-        const int v = base + lane < n ? ld_i(lists[slot & 1] + base + lane) : -1;
-        int rc = kStarOk;
-        if (v >= 0) {
-          SharedCand L;
-          rc = star_from_stars(P, v, L, lc);
-        }
-        fine = fine && rc != kStarDegenerate;
-        for (unsigned m = __ballot_sync(kFull, rc == kStarFull); m; m &= m - 1) {
-          const int u = __shfl_sync(kFull, v, __ffs(m) - 1);
-          if (!warp_from_stars(P, u, lc) && lane == 0) fine = star_alone(P, u, false, 0, true, lc) && fine;
-          __syncwarp();
-        }
-      }
-      if (!fine) atomicOr(cnt + (slot + 1) % 3, kStarGivenUp);
-      g.sync();
-      if (rounds <= 40) timeline(P, 1 + rounds);
-      touched = 0;
-      ++slot;
-      continue;
-    }
-    // few do: a warp makes one, then they check their neighbourhoods, until all agree
-    touched = stamp++;
+    // the stars that disagree, again, until their neighbourhoods agree: few are made
+    // by a warp each, many by a thread each
+    const unsigned ts = stamp++;
+    bool all_few = true;
     while (n > 0) {
       if (++rounds > kStarRounds) return false;
+      const bool many = n > kWarpStars * nwarps;
+      const int* list = lists[slot & 1];
       fine = true;
-      for (int i = gwarp; i < n; i += nwarps) {
-        const int v = ld_i(lists[slot & 1] + i);
-        warp_touch(P, v, touched);
-        if (!warp_from_stars(P, v, lc) && lane == 0) fine = star_alone(P, v, false, 0, true, lc) && fine;
-        __syncwarp();
-        warp_touch(P, v, touched);
+      if (many) {
+        all_few = false;
+        for (int base = gwarp * 32; base < n; base += stride) {
+          const int v = base + lane < n ? ld_i(list + base + lane) : -1;
+          int rc = kStarOk;
+          if (v >= 0) {
+            SharedCand L;
+            rc = star_from_stars(P, v, L, lc);
+          }
+          fine = fine && rc != kStarDegenerate;
+          for (unsigned m = __ballot_sync(kFull, rc == kStarFull); m; m &= m - 1) {
+            const int u = __shfl_sync(kFull, v, __ffs(m) - 1);
+            if (!warp_from_stars(P, u, lc) && lane == 0) fine = star_alone(P, u, false, 0, true, lc) && fine;
+            __syncwarp();
+          }
+        }
+      } else {
+        for (int i = gwarp; i < n; i += nwarps) {
+          const int v = ld_i(list + i);
+          warp_touch(P, v, ts);
+          if (!warp_from_stars(P, v, lc) && lane == 0) fine = star_alone(P, v, false, 0, true, lc) && fine;
+          __syncwarp();
+          warp_touch(P, v, ts);
+        }
       }
       if (!fine) atomicOr(cnt + (slot + 1) % 3, kStarGivenUp);
       g.sync();
+      if (rounds <= 40) timeline(P, 1 + rounds);
       ++slot;
+      if (2 * n > P.V_it) break;  // most were made: the next full check does as well
       cs = stamp++;
       if (gtid == 0) cnt[(slot + 1) % 3] = 0;
-      auto again = [&](int u) { star_list(P, u, cs, lists[slot & 1], cnt + slot % 3); };
-      for (int i = gwarp; i < n; i += nwarps) {
-        const int v = ld_i(lists[(slot - 1) & 1] + i);
-        int inner;
-        unsigned long long ranks;
-        warp_check(P, v, star_base(P, v).v0 + 4, true, again, &inner, &ranks);
+      int* next = lists[slot & 1];
+      int* count = cnt + slot % 3;
+      int inner;
+      unsigned long long ranks;
+      if (many) {
+        auto again = [&](int u) { __stcg(P.smark + u, cs); };
+        for (int i = spread_tid(); i < n; i += stride) {
+          const int v = ld_i(list + i);
+          star_check(P, v, star_base(P, v).v0 + 4, true, again, &inner, &ranks);
+        }
+        __syncwarp();
+        g.sync();
+        star_marked(P, cs, i0, i1, next, count);
+      } else {
+        auto again = [&](int u) { star_list(P, u, cs, next, count); };
+        for (int i = gwarp; i < n; i += nwarps) {
+          const int v = ld_i(list + i);
+          warp_check(P, v, star_base(P, v).v0 + 4, true, again, &inner, &ranks);
+        }
+        __syncwarp();
       }
-      __syncwarp();
       g.sync();
-      if (rounds <= 40) timeline(P, 1 + rounds);
-      n = ld_i(cnt + slot % 3);
+      n = ld_i(count);
       if (n >= kStarGivenUp || n < 0) return false;
+      if (n == 0) ++slot;
     }
-    ++slot;
+    touched = all_few ? ts : 0;
   }
   timeline(P, 44);
   int carry = sums[0];

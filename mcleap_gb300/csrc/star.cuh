@@ -33,9 +33,9 @@
 // (about 180 warp instructions per vertex and star with 12 of 32 lanes at work: rings
 // and candidate lists differ in length) and L2 latency.  The step's launch at sigma =
 // 0.1 x spacing, removal path before -> stars, GB300: 1,000 points 472 -> 92 us,
-// 10,000 points 586 -> 150 us, 1,000,000 points 1551 -> 1235 us; the precision-stress
+// 10,000 points 586 -> 155 us, 1,000,000 points 1551 -> 1260 us; the precision-stress
 // set of 500,000 (a third of it in clusters that move 1.4 of their spacings) 3332 ->
-// 2200 us.
+// 2130 us.
 //
 // The bodies are host/device code: the CPU can run them vertex by vertex.
 #pragma once
@@ -112,10 +112,9 @@ MCL_HD bool star_owned(int v, int w, int c4) { return w > v || w < c4; }
 // ---------------------------------------------------------------------------
 // Candidate lists: ids with their positions relative to v (rounded once: the
 // differences that the FP32 filters of orient2d and incircle start from with v
-// as the last point) and their pseudo-angles, in angular order.  One 16-byte
-// record each.
+// as the last point), in angular order.
 struct Cand {
-  float x, y, key;
+  float x, y;
   int id;
 };
 struct LocalCand {
@@ -127,15 +126,14 @@ struct LocalCand {
 
 enum : int { kStarOk = 0, kStarDegenerate = 1, kStarFull = 2 };
 
-// Candidate w at x, seen from pv.  The pseudo-angle in [0, 4] is monotone in the
-// angle up to 2e-6 (differences, quotient and sums rounded once each, the quotient
-// to 2 ulp); it is NaN when the two coincide.  Angles are counted from `from`, the
-// pseudo-angle of the first candidate, so that a ring comes in order.
-MCL_HD Cand star_cand(float2 pv, int w, float2 x, float from) {
-  Cand c;
-  c.x = fsub(x.x, pv.x);
-  c.y = fsub(x.y, pv.y);
-  c.id = w;
+// Candidate w at x, seen from pv.
+MCL_HD Cand star_cand(float2 pv, int w, float2 x) { return Cand{fsub(x.x, pv.x), fsub(x.y, pv.y), w}; }
+
+// Its pseudo-angle in [0, 4], monotone in the angle up to 2e-6 (differences,
+// quotient and sums rounded once each, the quotient to 2 ulp); NaN when it lies on v.
+// Angles are counted from `from`, the pseudo-angle of the first candidate, so that a
+// ring comes in order.
+MCL_HD float star_key(const Cand& c, float from) {
   const float s = fabsf(c.x) + fabsf(c.y);
 #if defined(__CUDA_ARCH__)
   const float t = __fdividef(c.y, s);  // s is at most 4e7, far below its limit
@@ -143,8 +141,7 @@ MCL_HD Cand star_cand(float2 pv, int w, float2 x, float from) {
   const float t = c.y / s;
 #endif
   const float k = (c.x >= 0.f ? (c.y >= 0.f ? t : 4.f + t) : 2.f - t) - from;
-  c.key = k < 0.f ? k + 4.f : k;
-  return c;
+  return k < 0.f ? k + 4.f : k;
 }
 constexpr float kStarSameKey = 8e-6f;
 
@@ -198,15 +195,17 @@ MCL_HD_NOINLINE int star_nearer(const float2* pos, int v, int u, int w) {
 // far: leave c out when it lies outside the circle of the entries beside it
 // (every wedge of the list is below 180 degrees).
 template <typename List>
-MCL_HD int star_insert(const KParams& P, int v, List& L, int& n, Cand c, bool far, LocalCounters& lc) {
-  if (!(c.key >= 0.f)) return kStarDegenerate;
+MCL_HD int star_insert(const KParams& P, int v, float from, List& L, int& n, Cand c, bool far, LocalCounters& lc) {
+  const float key = star_key(c, from);
+  if (!(key >= 0.f)) return kStarDegenerate;
   int j = n;
 #pragma unroll 1
   while (j > 0) {
     const Cand u = L.get(j - 1);
     if (u.id == c.id) return kStarOk;
-    bool before = u.key < c.key;
-    if (fabsf(u.key - c.key) < kStarSameKey) {
+    const float ku = star_key(u, from);
+    bool before = ku < key;
+    if (fabsf(ku - key) < kStarSameKey) {
       int s = star_cross(u, c);
       if (s == 2) {
         LocalCounters m = {0, 0, 0, 0, 0, 0, 0};
@@ -450,7 +449,7 @@ MCL_HD int star_corners(const KParams& P, int v, int v0, float from, List& L, in
   for (int i = f; i <= t; ++i, ++n) L.set(n, L.get(i));
 #pragma unroll 1
   for (int c = 0; c < 4; ++c)
-    if (star_insert(P, v, L, n, star_cand(pv, v0 + c, spos(P, v0 + c), from), false, lc) != kStarOk) return -1;
+    if (star_insert(P, v, from, L, n, star_cand(pv, v0 + c, spos(P, v0 + c)), false, lc) != kStarOk) return -1;
   return n;
 }
 
@@ -522,15 +521,12 @@ MCL_HD int star_from_mesh(const KParams& P, int v, bool keep, unsigned bad, List
     }
     if (keep) {
       if (n >= L.cap()) return kStarFull;
-      L.set(n++, Cand{0.f, 0.f, 0.f, x});
+      L.set(n++, Cand{0.f, 0.f, x});
       continue;
     }
-    Cand c = star_cand(pv, x, px, from);
-    if (n == 0) {
-      from = c.key;
-      c.key = c.key >= 0.f ? 0.f : c.key;  // NaN stays
-    }
-    const int rc = star_insert(P, v, L, n, c, false, lc);
+    const Cand c = star_cand(pv, x, px);
+    if (n == 0) from = star_key(c, 0.f);
+    const int rc = star_insert(P, v, from, L, n, c, false, lc);
     if (rc != kStarOk) return rc;
   }
   if (!round) return kStarDegenerate;
@@ -561,12 +557,9 @@ MCL_HD int star_from_stars(const KParams& P, int v, List& L, LocalCounters& lc) 
     x1 = entry(i + 1);
     if (x1 >= mb.v0 && x1 < mb.v1) p1 = spos(P, x1);
     if (i == me.n) far = !me.open && n >= 3;  // every wedge of the list is below 180 degrees
-    Cand c = star_cand(pv, x, px, from);
-    if (i == 0) {
-      from = c.key;
-      c.key = c.key >= 0.f ? 0.f : c.key;
-    }
-    const int rc = star_insert(P, v, L, n, c, far, lc);
+    const Cand c = star_cand(pv, x, px);
+    if (i == 0) from = star_key(c, 0.f);
+    const int rc = star_insert(P, v, from, L, n, c, far, lc);
     if (rc != kStarOk) return rc;
   }
   const int rc = star_finish(P, v, mb.v0, from, L, n, true, lc);
@@ -591,14 +584,14 @@ MCL_HD_NOINLINE int2 star_wedge(const int* srow, const int* sext, int ext_rows, 
   if (q.x & kRowExt) at = sext + (size_t)(q.y >= 0 && q.y < ext_rows ? q.y : 0) * kExtRow;
   if (n < 2 || n > ((q.x & kRowExt) ? kExtRow : kRowInline)) return make_int2(-1, -1);
   const float2 pw = pos[w];
-  const float k = star_cand(pw, v, pos[v], 0.f).key;
+  const float k = star_key(star_cand(pw, v, pos[v]), 0.f);
   int lo = -1, hi = -1, least = -1, most = -1;  // nearest keys below and above k, the extremes
   float klo = -1.f, khi = 9.f, kleast = 9.f, kmost = -1.f;
 #pragma unroll 1
   for (int i = 0; i < n; ++i) {
     const int u = sld(at + i);
     if (u < 0) return make_int2(-1, -1);
-    const float ku = star_cand(pw, u, pos[u], 0.f).key;
+    const float ku = star_key(star_cand(pw, u, pos[u]), 0.f);
     if (ku <= k && ku > klo) { klo = ku; lo = u; }
     if (ku > k && ku < khi) { khi = ku; hi = u; }
     if (ku < kleast) { kleast = ku; least = u; }
