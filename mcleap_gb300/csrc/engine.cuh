@@ -102,7 +102,7 @@ struct DevState {
   // published to ts[43..46] by a step without repair (a repair step keeps its
   // own marks there)
   unsigned long long tsmax[4];
-  // mcl_settle_moves: [0] last stamp used, [1..3] moves sent back per pass
+  // mcl_settle_moves: [0] last stamp used, [1..3] vertices listed per pass
   // (triple-buffered), [4] sent back by the last call, [5] status of the last call
   unsigned int settle[8];
 };
@@ -394,7 +394,7 @@ struct mcl_mesh {
   int* cbase;              // per component: first vertex (NULL for a plain mesh)
   int* cebase;             // per component: first edge (NULL for a plain mesh)
   // mcl_settle_moves
-  unsigned long long* table;  // hash table of positions, stamped entries
+  int* table;              // hash table of positions: the vertex in each slot
   int64_t table_size;
   int* smark;              // per vertex: stamp of the settle pass that found it coincident
   unsigned* smove;         // per mesh: stamp of the settle call that found a mover in it
