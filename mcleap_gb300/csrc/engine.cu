@@ -2989,7 +2989,7 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   A((void**)&m->cand, 4 * E);
   A((void**)&m->win, 4 * E);
   A((void**)&m->qmark, 4 * E);
-  A((void**)&m->efa, 8 * E);
+  A((void**)&m->efa, std::max(8 * E, 4 * kInbox * V));
   A((void**)&m->hard, 4 * E);
   A((void**)&m->wl[0], 4 * E);
   A((void**)&m->wl[1], 4 * E);
@@ -3215,7 +3215,7 @@ static KParams make_params(mcl_mesh* m, int mode) {
   P.sext = m->star + (int64_t)kRow * m->V;
   P.smark = reinterpret_cast<unsigned*>(m->star + star_mark_at(m->V));
   P.sblk = m->star + star_sums_at(m->V);
-  P.sinbox = P.sblk + 4 * kStarBlocks;
+  P.sinbox = reinterpret_cast<int*>(m->efa);
   P.srank = reinterpret_cast<unsigned long long*>(m->target);
   P.sbase = m->vloc;
   P.vcomp = m->vcomp;

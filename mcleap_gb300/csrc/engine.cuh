@@ -141,7 +141,7 @@ struct KParams {
   int* srow;               // star rows, kRow ints per vertex (star.cuh)
   int* sext;               // overflow rows
   unsigned* smark;         // per vertex: stamp of the last round that listed it
-  int* sinbox;             // kInbox ints per vertex: vertices to consider in the next round
+  int* sinbox;             // kInbox ints per vertex: vertices to consider in the next round (shares `efa`)
   int* sblk;               // per block: sums of the star check
   unsigned long long* srank;  // per vertex: ranks of its entries in their owners' rows (shares `target`)
   int* sbase;              // per vertex: own edges of the vertices before it (shares `vloc`)

@@ -61,9 +61,11 @@ constexpr int kStarRounds = 64;   // rounds of disagreeing stars before the remo
 MCL_HD int star_ext_rows(int64_t V) { return (int)(V / 64 + 64); }
 constexpr int kStarBlocks = 1024;  // most blocks of a launch (four sums each)
 // The scratch of such a mesh, in ints (all but the last part on 16 bytes): rows,
-// overflow rows, the block sums, the inboxes, a mark per vertex.
+// overflow rows, the block sums, a mark per vertex.  The inboxes share the flip rounds'
+// claims (`efa`): a launch that makes stars flips nothing unless they fail, and then
+// after the last of them has been read.
 MCL_HD int64_t star_sums_at(int64_t V) { return kRow * V + (int64_t)kExtRow * star_ext_rows(V); }
-MCL_HD int64_t star_mark_at(int64_t V) { return star_sums_at(V) + 4 * kStarBlocks + kInbox * V; }
+MCL_HD int64_t star_mark_at(int64_t V) { return star_sums_at(V) + 4 * kStarBlocks; }
 MCL_HD int64_t star_ints(int64_t V) { return star_mark_at(V) + V; }
 
 // What a phase reads it does not write, and a grid barrier lies between a phase
