@@ -54,6 +54,8 @@ enum Counter {
 
 constexpr int kTimeline = 48;
 
+constexpr float kSquare = 10000000.0f;  // the bounding square's corners are at +-this
+
 struct DevState {
   // working state of the running launch; the launch leaves it cleared
   int wl_count[2];         // edge work-list sizes
@@ -105,6 +107,9 @@ struct DevState {
   // mcl_settle_moves: [0] last stamp used, [1..3] vertices listed per pass
   // (triple-buffered), [4] sent back by the last call, [5] status of the last call
   unsigned int settle[8];
+  // mcl_mesh_build: where the points' Morton keys differ, and how many equal the one before
+  unsigned long long sort_mask;
+  int sort_ties;
 };
 
 enum MoveMode { MOVE_NONE = 0, MOVE_DISPLACE = 1, MOVE_INTEGRATE = 2 };
@@ -145,6 +150,7 @@ struct KParams {
   int* sblk;               // per block: sums of the star check
   unsigned long long* srank;  // per vertex: ranks of its entries in their owners' rows (shares `target`)
   int* sbase;              // per vertex: own edges of the vertices before it (shares `vloc`)
+  unsigned long long* skey;   // per vertex: Morton key, during a build (shares `vfree`)
   const int* vcomp;        // batches: mesh of a vertex, first vertex and first edge of a mesh (NULL: plain)
   const int* cbase;
   const int* cebase;

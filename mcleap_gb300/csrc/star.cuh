@@ -570,6 +570,57 @@ MCL_HD int star_from_stars(const KParams& P, int v, List& L, LocalCounters& lc) 
 }
 
 // ---------------------------------------------------------------------------
+// libmorton's m2D_e_LUT<uint_fast32_t,uint_fast32_t>(x, y) as the reference calls it:
+// each float truncated to an integer (two's complement for negative values), the low
+// 32 bits of x in the even bit positions, y in the odd ones.
+MCL_HD unsigned long long morton_spread(unsigned long long w) {
+  w &= 0xFFFFFFFFull;
+  w = (w | (w << 16)) & 0x0000FFFF0000FFFFull;
+  w = (w | (w << 8)) & 0x00FF00FF00FF00FFull;
+  w = (w | (w << 4)) & 0x0F0F0F0F0F0F0F0Full;
+  w = (w | (w << 2)) & 0x3333333333333333ull;
+  w = (w | (w << 1)) & 0x5555555555555555ull;
+  return w;
+}
+MCL_HD unsigned long long morton_cell(unsigned x, unsigned y) {
+  return morton_spread(x) | morton_spread(y) << 1;
+}
+MCL_HD unsigned long long morton_key(float x, float y) {
+  return morton_cell((unsigned)(long long)x, (unsigned)(long long)y);
+}
+
+// The points of an aligned square cell are consecutive in the Morton order, so a cell
+// is found by bisection.  The cell around v is the smallest that holds kOrderNear
+// consecutive points with v among them: its size follows the density of the points.
+
+MCL_HD unsigned long long order_key(const KParams& P, int v) { return P.skey[v]; }
+// First vertex in [lo, hi] whose key is at least k (hi + 1: none).
+MCL_HD int order_bisect(const KParams& P, unsigned long long k, int lo, int hi) {
+  int n = hi - lo + 1;
+  while (n > 0) {
+    const int h = n >> 1;
+    if (order_key(P, lo + h) < k) {
+      lo += h + 1;
+      n -= h + 1;
+    } else {
+      n = h;
+    }
+  }
+  return lo;
+}
+constexpr int kOrderNear = 3;
+constexpr int kOrderCell = 3;  // candidates from each of the nine cells
+// Side of that cell as a power of two, for window k of kOrderNear consecutive points.
+MCL_HD int order_cell(const KParams& P, int v, int k, int lo, int hi) {
+  const int a = v - k, b = a + kOrderNear - 1;
+  if (a < lo || b > hi) return 32;
+  const unsigned long long d = order_key(P, a) ^ order_key(P, b);
+  int bits = 0;
+  while (bits < 32 && d >> (2 * bits)) ++bits;
+  return bits;
+}
+
+// ---------------------------------------------------------------------------
 // x is left for v to consider when it makes its star again.
 MCL_HD void star_tell(const KParams& P, int v, int x, int c4) {
   if (v < c4 || x == v) return;
