@@ -29,9 +29,13 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
+
+#include <unistd.h>
 
 #include "engine.cuh"
 #include "star.cuh"
@@ -3213,12 +3217,9 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 void free_mesh(mcl_mesh* m) {
   if (!m) return;
-  void* ptrs[] = {m->pos[0], m->pos[1], m->ev, m->en, m->vhe, m->vfix, m->cand, m->win, m->qmark, m->efa, m->hard,
-                  m->wl[0], m->wl[1], m->vl[0], m->vl[1], m->vmark, m->claim, m->vfree, m->vhint,
-                  m->vaux, m->vloc, m->vlocf, m->target, m->star, m->cebase, m->vprev, m->vl2, m->dstage, m->scratch, m->st,
-                  m->vcomp, m->vroot, m->cbase, m->table, m->smark, m->smove, m->fnew, m->act_dev,
-                  m->bg_cell, m->bg_src, m->bg_perm, m->bg_pos, m->bg_count, m->bg_start, m->bg_cursor,
-                  m->bg_tmp, m->bg_par, m->aos_tmp};
+  void* ptrs[] = {m->slab, m->cebase, m->vprev, m->vl2, m->vcomp, m->vroot, m->cbase, m->table, m->smark, m->smove,
+                  m->fnew, m->act_dev, m->bg_cell, m->bg_src, m->bg_perm, m->bg_pos, m->bg_count, m->bg_start,
+                  m->bg_cursor, m->bg_tmp, m->bg_par, m->aos_tmp};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (m->dstage2) cudaFree(m->dstage2);
@@ -3231,7 +3232,10 @@ void free_mesh(mcl_mesh* m) {
       cudaEventDestroy(m->ev_used[i]);
     }
   }
-  if (m->st_host) cudaFreeHost(m->st_host);
+  if (m->st_host) {
+    if (m->counts_host) cudaHostUnregister(m->st_host);
+    std::free(m->st_host);
+  }
   if (m->act_host) cudaFreeHost(m->act_host);
   if (m->bg_par_host) cudaFreeHost(m->bg_par_host);
   delete[] m->comp_host;
@@ -3264,9 +3268,13 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   m->T = 2 * (V - 4) + 2;
   m->cur = 0;
   m->valid_cur = true;
-  cudaError_t e = cudaSuccess;
+  // one allocation, each array on 256 bytes; those that start as zeros lie together, and
+  // those that start as -1
+  size_t at = 0;
+  std::vector<std::pair<void**, size_t>> parts;
   auto A = [&](void** p, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+    parts.emplace_back(p, at);
+    at += (bytes + 255) / 256 * 256;
   };
   A((void**)&m->pos[0], 8 * V);
   A((void**)&m->pos[1], 8 * V);
@@ -3274,47 +3282,50 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   A((void**)&m->en, 16 * E);
   A((void**)&m->vhe, 4 * V);
   A((void**)&m->vfix, V);
-  A((void**)&m->cand, 4 * E);
-  A((void**)&m->win, 4 * E);
-  A((void**)&m->qmark, 4 * E);
   A((void**)&m->efa, std::max(8 * E, 4 * kInbox * V));
   A((void**)&m->hard, 4 * E);
   A((void**)&m->wl[0], 4 * E);
   A((void**)&m->wl[1], 4 * E);
   A((void**)&m->vl[0], 4 * V);
   A((void**)&m->vl[1], 4 * V);
-  A((void**)&m->vmark, 4 * V);
-  A((void**)&m->claim, 8 * 2 * E);
   A((void**)&m->vfree, 12 * V);
-  A((void**)&m->vhint, 4 * V);
-  A((void**)&m->vaux, 4 * V);
   A((void**)&m->vloc, 4 * V);
   A((void**)&m->vlocf, 4 * V);
   A((void**)&m->target, 8 * V);
-  A((void**)&m->star, 4 * star_ints(V));
   A((void**)&m->dstage, 8 * V);
+  const size_t ones = at;
+  A((void**)&m->vaux, 4 * V);
+  A((void**)&m->vhint, 4 * V);
+  const size_t zeros = at + 4 * star_mark_at(V);  // the marks end the star scratch
+  A((void**)&m->star, 4 * star_ints(V));
+  A((void**)&m->cand, 4 * E);
+  A((void**)&m->win, 4 * E);
+  A((void**)&m->qmark, 4 * E);
+  A((void**)&m->claim, 8 * 2 * E);
+  A((void**)&m->vmark, 4 * V);
   A((void**)&m->scratch, kScratchBytes);
   A((void**)&m->st, sizeof(DevState));
-  // the mirror of the device state, and behind it the counts that queries write
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&m->st_host, sizeof(DevState) + 64);
+  cudaError_t e = cudaMalloc((void**)&m->slab, at);
+  if (e == cudaSuccess)
+    for (const auto& [p, off] : parts) *p = m->slab + off;
+  // the mirror of the device state, and behind it the counts that queries write: pages
+  // of the host's, pinned in place
+  if (e == cudaSuccess) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), bytes = (sizeof(DevState) + 64 + page - 1) / page * page;
+    m->st_host = static_cast<DevState*>(std::aligned_alloc(page, bytes));
+    e = m->st_host ? cudaHostRegister(m->st_host, bytes, cudaHostRegisterMapped) : cudaErrorMemoryAllocation;
+  }
   if (e == cudaSuccess) m->counts_host = reinterpret_cast<unsigned long long*>(m->st_host + 1);
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&m->counts_dev, m->counts_host, 0);
   if (e != cudaSuccess) {
+    (void)cudaGetLastError();
     free_mesh(m);
     return cuda_fail(e, "cudaMalloc(mesh)");
   }
-  e = cudaMemset(m->cand, 0, 4 * E);
-  if (e == cudaSuccess) e = cudaMemset(m->win, 0, 4 * E);
-  if (e == cudaSuccess) e = cudaMemset(m->qmark, 0, 4 * E);
-  if (e == cudaSuccess) e = cudaMemset(m->claim, 0, 16 * E);
-  if (e == cudaSuccess) e = cudaMemset(m->vaux, 0xff, 4 * V);
-  if (e == cudaSuccess) e = cudaMemset(m->vhint, 0xff, 4 * V);
-  if (e == cudaSuccess) e = cudaMemset(m->vmark, 0, 4 * V);
-  if (e == cudaSuccess) e = cudaMemset(m->scratch, 0, kScratchBytes);
-  if (e == cudaSuccess) e = cudaMemset(m->star + star_mark_at(V), 0, 4 * V);
-  DevState s;
-  std::memset(&s, 0, sizeof(s));
-  s.epoch = 1;
-  if (e == cudaSuccess) e = cudaMemcpy(m->st, &s, sizeof(s), cudaMemcpyHostToDevice);
+  e = cudaMemsetAsync(m->slab + zeros, 0, at - zeros, 0);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->slab + ones, 0xff, zeros - 4 * star_mark_at(V) - ones, 0);
+  const unsigned epoch = 1;
+  if (e == cudaSuccess) e = cudaMemcpy(&m->st->epoch, &epoch, sizeof(epoch), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     free_mesh(m);
     return cuda_fail(e, "mesh init");

@@ -345,6 +345,7 @@ __device__ __forceinline__ bool flip_edge(const KParams& P, int e) {
 struct mcl_mesh {
   int device;
   int64_t V, E, T;
+  char* slab;              // the arrays of every mesh, in one allocation (alloc_mesh)
   int cur;                 // index of the current position buffer
   bool valid_cur;          // pos[cur] is the last validated state
   float2* pos[2];
@@ -378,9 +379,10 @@ struct mcl_mesh {
   mcl_step_stats* stats_dev;  // [2] published counters of the pipelined steps
   int stage_idx;
   unsigned long long* scratch;  // small device scratch for query counters (kScratchBytes)
-  unsigned long long* counts_host;  // pinned, device-visible: counts of the last counted queries
+  unsigned long long* counts_host;  // behind st_host: counts of the last counted queries
+  unsigned long long* counts_dev;   // the same, as the device sees them
   mcl::DevState* st;
-  mcl::DevState* st_host;  // pinned mirror
+  mcl::DevState* st_host;  // pinned mirror (own pages, registered)
   int coop_blocks;         // k_step grid
   int repair_blocks;       // k_repair grid
   int coop_threads;

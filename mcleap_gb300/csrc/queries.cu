@@ -924,7 +924,8 @@ int launch_one_ring(mcl_mesh* m, const int* verts, int64_t n, int layout, int ma
   unsigned long long* host = truncated ? m->counts_host + kHostRing : nullptr;
   auto kernel = layout == MCL_LAYOUT_COLUMN ? k_one_ring<false> : k_one_ring<true>;
   kernel<<<blocks, kRingThreads, 0, s>>>(mesh_view(m), verts, (int)n, max_ring, out, m->vfix, delaunay,
-                                         host ? m->scratch + kCellRing : nullptr, host);
+                                         host ? m->scratch + kCellRing : nullptr,
+                                         host ? m->counts_dev + kHostRing : nullptr);
   QCK(cudaGetLastError());
   return wait_count(host, s, truncated);
 }
@@ -938,8 +939,8 @@ int launch_mesh_frnn(mcl_mesh* m, const int* verts, int64_t n, float r2, const f
   }
   unsigned long long* host = overflow ? m->counts_host + kHostFrnn : nullptr;
   k_mesh_frnn<<<(unsigned)((n + kFrnnWarps - 1) / kFrnnWarps), 32 * kFrnnWarps, 0, s>>>(
-      mesh_view(m), verts, (int)n, r2, layout, max_frnn, out, host ? m->scratch + kCellFrnn : nullptr, host, rcomp,
-      rcomp ? m->vcomp : nullptr);
+      mesh_view(m), verts, (int)n, r2, layout, max_frnn, out, host ? m->scratch + kCellFrnn : nullptr,
+      host ? m->counts_dev + kHostFrnn : nullptr, rcomp, rcomp ? m->vcomp : nullptr);
   QCK(cudaGetLastError());
   return wait_count(host, s, overflow);
 }
