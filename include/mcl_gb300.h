@@ -259,7 +259,7 @@ int mcl_grid_mean_occupancy(mcl_grid* g, float* mean_host);
  * allocator).  No counterpart in the reference: it does what mcl_grid_create +
  * mcl_grid_update + mcl_grid_frnn do, but allocates nothing and leaves pos_dev
  * untouched.  Its scratch is one fixed array in the library's device image
- * (5.3 MB held on every GPU that loads the library until exit); limits: n <=
+ * (6.3 MB held on every GPU that loads the library until exit); limits: n <=
  * 262144 points and at most 262144 cell-table entries, else MCL_ERR_CAPACITY.
  * Outputs (caller-owned device buffers): sorted_pos_dev[n] = positions in cell
  * order, perm_dev[n] = sorted slot of input point i, counts_dev[n] and

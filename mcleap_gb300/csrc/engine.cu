@@ -3218,8 +3218,8 @@ int cuda_fail(cudaError_t e, const char* what) {
 void free_mesh(mcl_mesh* m) {
   if (!m) return;
   void* ptrs[] = {m->slab, m->cebase, m->vprev, m->vl2, m->vcomp, m->vroot, m->cbase, m->table, m->smark, m->smove,
-                  m->fnew, m->act_dev, m->bg_cell, m->bg_src, m->bg_perm, m->bg_pos, m->bg_count, m->bg_start,
-                  m->bg_cursor, m->bg_tmp, m->bg_par, m->aos_tmp};
+                  m->fnew, m->act_dev, m->bg_cell, m->bg_src, m->bg_rank, m->bg_bucket, m->bg_pos, m->bg_count,
+                  m->bg_start, m->bg_local, m->bg_pre, m->bg_par, m->aos_tmp};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (m->dstage2) cudaFree(m->dstage2);

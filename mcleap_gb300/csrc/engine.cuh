@@ -411,12 +411,13 @@ struct mcl_mesh {
   // mcl_batch_frnn_grid: one uniform grid per mesh, cells of all meshes in one table
   int* bg_cell;            // per vertex: its cell (-1: bounding corner)
   int* bg_src;             // per sorted slot: vertex
-  int* bg_perm;            // per vertex: sorted slot
+  int* bg_rank;            // per vertex: its place in its cell by arrival
+  int* bg_bucket;          // per slot: vertex, in order of arrival
   float2* bg_pos;          // per sorted slot: position
   int* bg_count;           // per cell
   int* bg_start;
-  int* bg_cursor;
-  int* bg_tmp;             // scan scratch
+  int* bg_local;           // per cell: start within its scan block
+  int* bg_pre;             // per scan block: points before it
   int4* bg_par;            // per mesh: {cell size bits, cells per side, first cell, 0}
   int4* bg_par_host;       // pinned copy of the uploaded grid parameters
   int64_t bg_cap;          // cells the tables hold
