@@ -560,7 +560,8 @@ __device__ __forceinline__ int cell_id(const GridView& G, int x, int y) {
 // counts the smaller indices of its cell, which gives its slot.  Nothing is sorted in
 // place, so no lone thread orders a crowded cell.  Bound by launches below 100,000
 // points and by scattered atomics and stores above (1,000,000 points, 2.4 per cell:
-// 57 -> 48 us; a pass over 10,000 points takes 30 us less; the ten launches before had a scan in three, a copy of the starts as
+// 57 -> 48 us; a pass over 10,000 points takes 30 us
+// less; the ten launches before had a scan in three, a copy of the starts as
 // cursors with a second round of atomics, an insertion sort per cell and a gather).
 constexpr int kScanThreads = 1024;
 constexpr int kScanCells = 4 * kScanThreads;  // cells per block of the scan
@@ -719,29 +720,189 @@ __global__ void k_scan_add(int* out, const int* block_prefix, int64_t n) {
 // order, gridCount2d.h:263-296).  Distances use the reference formula
 // fl(fl(dx*dx) + fl(dy*dy)) <= fl(r*r) without FMA; periodic grids take the
 // minimum image (|d| > L/2 -> d -= copysign(L, d)).  A candidate is tested
-// without branches: its sorted index is written to the thread's shared row at
-// slot nf and nf advances on a hit (a range takes this path only when the row
-// has room for all of it).  Rows hold up to kStageCap ids and are flushed one
-// warp per row (coalesced), ids and rows mapped through src when given;
-// entries past kStageCap go straight to global memory.
+// without branches: its distance from i in the order is written to the thread's
+// shared row at slot nf and nf advances on a hit (a range takes this path only when
+// the row has room for all of it and 16 bits for the distance).  Rows hold up to
+// kStageCap neighbours and are flushed by their own warp one after the other
+// (coalesced), ids and rows mapped through src when given; what does not fit goes
+// straight to global memory.
+// Bound by the latency of the candidates' loads (some 50 per point at r = 1.92 cells of
+// 2.4 points): rows of 16 bits leave the L1 twice the room and let 40 warps reside
+// instead of 32, and both coordinates of a candidate share an instruction.  r = 3 x
+// spacing, 1,000,000 points, periodic: 176 -> 131 us (rows of 32 bits: 174).
 constexpr int kStageCap = 48;
 constexpr int kFrnnThreads = 128;
+constexpr int kFrnnBlocks = 12;  // per SM: 40 registers (14 blocks spill: 152 us for 131; 10: 139)
+
+// To 2 ulp, where a margin of 1e-4 follows.
+__device__ __forceinline__ float near_sqrt(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// Two floats in one register pair: both lanes rounded to nearest, as one at a time.
+__device__ __forceinline__ unsigned long long pair_of(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ unsigned long long pair_add(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// fl(fl(x x) + fl(y y))
+__device__ __forceinline__ float pair_norm2(unsigned long long d) {
+  float x, y;
+  asm("{\n\t.reg .b64 q;\n\tmul.rn.f32x2 q, %2, %2;\n\tmov.b64 {%0, %1}, q;\n\t}" : "=f"(x), "=f"(y) : "l"(d));
+  return __fadd_rn(x, y);
+}
+
+// The candidates b .. e - 1 within r of a point, from slot nf of its row on.  The
+// differences have the opposite sign of the reference's (candidate - point, minus the
+// shift): rounding is symmetric and they are squared.
+template <bool kShift>
+__device__ __forceinline__ int near_range(const float2* __restrict__ pos, int b, int e, unsigned long long minus_p,
+                                          unsigned long long minus_shift, float r2, int i, short* mine, int nf) {
+  const unsigned long long* at = reinterpret_cast<const unsigned long long*>(pos);
+#pragma unroll 4
+  for (int j = b; j < e; ++j) {
+    unsigned long long d = pair_add(at[j], minus_p);
+    if (kShift) d = pair_add(d, minus_shift);
+    const bool hit = (pair_norm2(d) <= r2) & (j != i);
+    mine[nf] = (short)(j - i);
+    nf += hit ? 1 : 0;
+  }
+  return nf;
+}
+
+// How a grid's rows end: points beyond the domain clamped into the border cells; the
+// minimum image by row segment (see k_grid_frnn); the minimum image per candidate.
+enum : int { kNearClamp = 0, kNearSegment = 1, kNearWrap = 2 };
+
+struct NearQuery {
+  float r, ix, iy, Lx, Ly;  // radius, 1 / cell, domain
+  int max_nb, scap;         // neighbours wanted, and how many of them are staged
+};
+
+// The neighbours of point i into its stage row (past scap into direct); how many.
+template <int kMode>
+__device__ __forceinline__ int near_rows(const GridView& G, const NearQuery& Q, const float2* __restrict__ pos,
+                                         const int* __restrict__ start, float2 p, int i, short* mine, int* direct,
+                                         const int* __restrict__ src) {
+  int nf = 0;
+  const float r = Q.r, r2 = __fmul_rn(r, r);
+  const float hx = 0.5f * Q.Lx, hy = 0.5f * Q.Ly;
+  const float mx = 1e-3f * G.cx + 1e-5f * (fabsf(p.x) + fabsf(G.minx) + r);
+  const float my = 1e-3f * G.cy + 1e-5f * (fabsf(p.y) + fabsf(G.miny) + r);
+  const float px = p.x - G.minx, py = p.y - G.miny;
+  const unsigned long long minus_p = pair_of(-p.x, -p.y);
+  int ylo = (int)floorf(fmaxf(fminf((py - r - my) * Q.iy, 1e9f), -1e9f));
+  int yhi = (int)floorf(fmaxf(fminf((py + r + my) * Q.iy, 1e9f), -1e9f));
+  if (kMode == kNearClamp) {
+    ylo = ylo < 0 ? 0 : (ylo >= G.ny ? G.ny - 1 : ylo);
+    yhi = yhi < 0 ? 0 : (yhi >= G.ny ? G.ny - 1 : yhi);
+  } else if (kMode == kNearWrap && yhi - ylo + 1 > G.ny) {
+    ylo = 0; yhi = G.ny - 1;  // the disk covers every row: visit each once
+  }
+  for (int yy = ylo; yy <= yhi; ++yy) {
+    // vertical distance from p to the row's slab (0 inside), minus the margin;
+    // without wrap the border rows also hold the points clamped into them,
+    // so their slabs extend to infinity
+    float slo = yy * G.cy, shi = slo + G.cy;
+    if (kMode == kNearClamp) {
+      if (yy == 0) slo = -INFINITY;
+      if (yy == G.ny - 1) shi = INFINITY;
+    }
+    const float dym = fmaxf(fmaxf(slo - py, py - shi) - my, 0.f);
+    const float hw = (kMode == kNearWrap && yhi - ylo + 1 >= G.ny) ? r + mx
+                                                                   : near_sqrt(fmaxf(r2 - dym * dym, 0.f)) * 1.0001f + mx;
+    int xlo = (int)floorf(fmaxf(fminf((px - hw) * Q.ix, 1e9f), -1e9f));
+    int xhi = (int)floorf(fmaxf(fminf((px + hw) * Q.ix, 1e9f), -1e9f));
+    int y = yy;
+    float xs = 0.f, ys = 0.f;
+    if (kMode == kNearSegment) {
+      if (y < 0) { y += G.ny; ys = Q.Ly; }
+      else if (y >= G.ny) { y -= G.ny; ys = -Q.Ly; }
+    } else if (kMode == kNearWrap) {
+      y %= G.ny;
+      if (y < 0) y += G.ny;
+      if (xhi - xlo + 1 > G.nx) { xlo = 0; xhi = G.nx - 1; }
+    } else {
+      xlo = xlo < 0 ? 0 : (xlo >= G.nx ? G.nx - 1 : xlo);
+      xhi = xhi < 0 ? 0 : (xhi >= G.nx ? G.nx - 1 : xhi);
+    }
+    const int* row = start + y * G.nx;
+    // [xlo, xhi] in stencil order: from its wrapped start to the end of the row, then
+    // on from cell 0.  By segment, cells left of 0 are the row's end (+Lx), right of
+    // nx - 1 its start (-Lx).
+    int sa = xlo, more = -1;
+    if (kMode == kNearSegment) {
+      if (xlo < 0) { sa += G.nx; xs = Q.Lx; }
+    } else if (kMode == kNearWrap) {
+      sa = (xlo % G.nx + G.nx) % G.nx;
+    }
+    int sb = sa + (xhi - xlo);
+    if (kMode != kNearClamp && sb >= G.nx) {
+      more = sb - G.nx;
+      sb = G.nx - 1;
+    }
+    for (;;) {
+      const int b = __ldg(row + sa), e = __ldg(row + sb + 1);
+      const bool fits = nf + (e - b) <= Q.scap && b - i >= -32768 && e - i <= 32768;
+      if (fits && kMode == kNearWrap) {
+#pragma unroll 4
+        for (int j = b; j < e; ++j) {
+          const float2 o = pos[j];
+          float dx = __fsub_rn(p.x, o.x), dy = __fsub_rn(p.y, o.y);
+          dx = fabsf(dx) > hx ? __fsub_rn(dx, copysignf(Q.Lx, dx)) : dx;
+          dy = fabsf(dy) > hy ? __fsub_rn(dy, copysignf(Q.Ly, dy)) : dy;
+          const bool hit = (__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= r2) & (j != i);
+          mine[nf] = (short)(j - i);
+          nf += hit ? 1 : 0;
+        }
+      } else if (fits) {
+        if (kMode == kNearSegment && (xs != 0.f || ys != 0.f))
+          nf = near_range<true>(pos, b, e, minus_p, pair_of(-xs, -ys), r2, i, mine, nf);
+        else
+          nf = near_range<false>(pos, b, e, minus_p, 0, r2, i, mine, nf);
+      } else {
+        for (int j = b; j < e; ++j) {
+          const float2 o = pos[j];
+          float dx = __fsub_rn(p.x, o.x), dy = __fsub_rn(p.y, o.y);
+          if (kMode != kNearClamp) {
+            dx = fabsf(dx) > hx ? __fsub_rn(dx, copysignf(Q.Lx, dx)) : dx;
+            dy = fabsf(dy) > hy ? __fsub_rn(dy, copysignf(Q.Ly, dy)) : dy;
+          }
+          if ((__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= r2) & (j != i)) {
+            const bool near = j - i >= -32768 && j - i < 32768;
+            if (nf < Q.scap) mine[nf] = near ? (short)(j - i) : (short)0;  // 0: written already
+            if (nf < Q.max_nb && (nf >= Q.scap || !near)) direct[nf] = src ? __ldg(src + j) : j;
+            ++nf;
+          }
+        }
+      }
+      if (kMode == kNearClamp || more < 0) break;
+      sa = 0;
+      sb = more;
+      more = -1;
+      xs = kMode == kNearSegment && xs == 0.f ? -Q.Lx : 0.f;
+    }
+  }
+  return nf;
+}
 
 template <bool kPeriodic>
-__global__ void __launch_bounds__(kFrnnThreads) k_grid_frnn(GridView G, int n, const float2* __restrict__ pos,
-                                                           const int* __restrict__ start,
-                                                           const int* __restrict__ count, float r, float Lx,
-                                                           float Ly, int max_nb, int* __restrict__ counts,
+__global__ void __launch_bounds__(kFrnnThreads, kFrnnBlocks) k_grid_frnn(GridView G, NearQuery Q, int n,
+                                                           const float2* __restrict__ pos,
+                                                           const int* __restrict__ start, int* __restrict__ counts,
                                                            int* __restrict__ ids, unsigned long long* overflow,
                                                            const int* __restrict__ src,
                                                            const int* __restrict__ outside, int wrap_by_segment) {
-  __shared__ int stage[kFrnnThreads * (kStageCap + 1)];
-  __shared__ int cnts[kFrnnThreads];
-  const int t = threadIdx.x, row0 = blockIdx.x * kFrnnThreads, i = row0 + t;
-  int* mine = stage + t * (kStageCap + 1);
-  const int scap = max_nb < kStageCap ? max_nb : kStageCap;
-  int nf = 0;
-  const float r2 = __fmul_rn(r, r);
+  __shared__ short stage[kFrnnThreads * (kStageCap + 1)];
+  const int t = threadIdx.x, lane = t & 31, i = blockIdx.x * kFrnnThreads + t;
+  short* mine = stage + t * (kStageCap + 1);
+  int nf = 0, row = -1;
   // Minimum image by segment: with every point inside the domain and the
   // stencil well under half the domain (checked by the caller), a candidate's
   // |dx| exceeds half the domain exactly when its cell was reached across the
@@ -750,128 +911,33 @@ __global__ void __launch_bounds__(kFrnnThreads) k_grid_frnn(GridView G, int n, c
   const bool seg = kPeriodic && wrap_by_segment && outside && __ldg(outside) == 0;
   if (i < n) {
     const float2 p = pos[i];
-    const int row = src ? __ldg(src + i) : i;
-    int* direct = ids + (size_t)row * max_nb;
-    const float hx = 0.5f * Lx, hy = 0.5f * Ly;
-    const float ix = 1.0f / G.cx, iy = 1.0f / G.cy;
-    const float mx = 1e-3f * G.cx + 1e-5f * (fabsf(p.x) + fabsf(G.minx) + r);
-    const float my = 1e-3f * G.cy + 1e-5f * (fabsf(p.y) + fabsf(G.miny) + r);
-    const float px = p.x - G.minx, py = p.y - G.miny;
-    int ylo = (int)floorf(fmaxf(fminf((py - r - my) * iy, 1e9f), -1e9f));
-    int yhi = (int)floorf(fmaxf(fminf((py + r + my) * iy, 1e9f), -1e9f));
-    if (!kPeriodic) {
-      ylo = ylo < 0 ? 0 : (ylo >= G.ny ? G.ny - 1 : ylo);
-      yhi = yhi < 0 ? 0 : (yhi >= G.ny ? G.ny - 1 : yhi);
-    } else if (yhi - ylo + 1 > G.ny) {
-      ylo = 0; yhi = G.ny - 1;  // the disk covers every row: visit each once
-    }
-    for (int yy = ylo; yy <= yhi; ++yy) {
-      // vertical distance from p to the row's slab (0 inside), minus the margin;
-      // without wrap the border rows also hold the points clamped into them,
-      // so their slabs extend to infinity
-      float slo = yy * G.cy, shi = slo + G.cy;
-      if (!kPeriodic) {
-        if (yy == 0) slo = -INFINITY;
-        if (yy == G.ny - 1) shi = INFINITY;
-      }
-      const float dym = fmaxf(fmaxf(slo - py, py - shi) - my, 0.f);
-      const float hw = (kPeriodic && yhi - ylo + 1 >= G.ny) ? r + mx : sqrtf(fmaxf(r2 - dym * dym, 0.f)) * 1.0001f + mx;
-      int xlo = (int)floorf(fmaxf(fminf((px - hw) * ix, 1e9f), -1e9f));
-      int xhi = (int)floorf(fmaxf(fminf((px + hw) * ix, 1e9f), -1e9f));
-      int y = yy;
-      float ys = 0.f;
-      if (kPeriodic && seg) {
-        if (y < 0) { y += G.ny; ys = Ly; }
-        else if (y >= G.ny) { y -= G.ny; ys = -Ly; }
-      } else if (kPeriodic) {
-        y %= G.ny;
-        if (y < 0) y += G.ny;
-        if (xhi - xlo + 1 > G.nx) { xlo = 0; xhi = G.nx - 1; }
-      } else {
-        xlo = xlo < 0 ? 0 : (xlo >= G.nx ? G.nx - 1 : xlo);
-        xhi = xhi < 0 ? 0 : (xhi >= G.nx ? G.nx - 1 : xhi);
-      }
-      const int base = y * G.nx;
-#pragma unroll 1
-      for (int sgi = 0; sgi < 2; ++sgi) {
-        int sa, sb;
-        float xs = 0.f;
-        if (kPeriodic && seg) {
-          // cells left of 0 are the row's end (+Lx), right of nx-1 its start (-Lx)
-          const int s0 = xlo < 0 ? xlo + G.nx : xlo, last = s0 + (xhi - xlo);
-          if (sgi == 0) { sa = s0; sb = last < G.nx ? last : G.nx - 1; xs = xlo < 0 ? Lx : 0.f; }
-          else { if (last < G.nx) continue; sa = 0; sb = last - G.nx; xs = xlo < 0 ? 0.f : -Lx; }
-        } else if (kPeriodic) {
-          // [xlo, xhi] (at most nx cells) in stencil order: from the wrapped
-          // start to the end of the row, then on from cell 0
-          const int s0 = (xlo % G.nx + G.nx) % G.nx, last = s0 + (xhi - xlo);
-          if (sgi == 0) { sa = s0; sb = last < G.nx ? last : G.nx - 1; }
-          else if (sgi == 1) { if (last < G.nx) continue; sa = 0; sb = last - G.nx; }
-          else continue;
-        } else {
-          if (sgi != 0) continue;
-          sa = xlo; sb = xhi;
-        }
-        const int b = __ldg(start + base + sa);
-        const int e = __ldg(start + base + sb) + __ldg(count + base + sb);
-        if (seg && nf + (e - b) <= scap) {
-#pragma unroll 4
-          for (int j = b; j < e; ++j) {
-            const float2 o = pos[j];
-            const float dx = __fadd_rn(__fsub_rn(p.x, o.x), xs), dy = __fadd_rn(__fsub_rn(p.y, o.y), ys);
-            const bool hit = (__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= r2) & (j != i);
-            mine[nf] = j;
-            nf += hit ? 1 : 0;
-          }
-        } else if (nf + (e - b) <= scap) {
-#pragma unroll 4
-          for (int j = b; j < e; ++j) {
-            const float2 o = pos[j];
-            float dx = __fsub_rn(p.x, o.x), dy = __fsub_rn(p.y, o.y);
-            if (kPeriodic) {
-              dx = fabsf(dx) > hx ? __fsub_rn(dx, copysignf(Lx, dx)) : dx;
-              dy = fabsf(dy) > hy ? __fsub_rn(dy, copysignf(Ly, dy)) : dy;
-            }
-            const bool hit = (__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= r2) & (j != i);
-            mine[nf] = j;
-            nf += hit ? 1 : 0;
-          }
-        } else {
-          for (int j = b; j < e; ++j) {
-            const float2 o = pos[j];
-            float dx = __fsub_rn(p.x, o.x), dy = __fsub_rn(p.y, o.y);
-            if (kPeriodic) {
-              dx = fabsf(dx) > hx ? __fsub_rn(dx, copysignf(Lx, dx)) : dx;
-              dy = fabsf(dy) > hy ? __fsub_rn(dy, copysignf(Ly, dy)) : dy;
-            }
-            if ((__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= r2) & (j != i)) {
-              if (nf < scap) mine[nf] = j;
-              else if (nf < max_nb) direct[nf] = src ? __ldg(src + j) : j;
-              ++nf;
-            }
-          }
-        }
-      }
-    }
-    counts[row] = nf < max_nb ? nf : max_nb;
-    if (nf > max_nb) atomicAdd(overflow, 1ull);
+    row = src ? __ldg(src + i) : i;
+    int* direct = ids + (size_t)row * Q.max_nb;
+    if (!kPeriodic) nf = near_rows<kNearClamp>(G, Q, pos, start, p, i, mine, direct, src);
+    else if (seg) nf = near_rows<kNearSegment>(G, Q, pos, start, p, i, mine, direct, src);
+    else nf = near_rows<kNearWrap>(G, Q, pos, start, p, i, mine, direct, src);
+    counts[row] = nf < Q.max_nb ? nf : Q.max_nb;
+    if (nf > Q.max_nb) atomicAdd(overflow, 1ull);
   }
-  cnts[t] = nf < scap ? nf : scap;
-  __syncthreads();
-  const int lane = t & 31;
-  for (int rr = t >> 5; rr < kFrnnThreads && row0 + rr < n; rr += kFrnnThreads / 32) {
-    const int cr = cnts[rr];
-    const int row = src ? __ldg(src + row0 + rr) : row0 + rr;
-    int* dst = ids + (size_t)row * max_nb;
-    const int* from = stage + rr * (kStageCap + 1);
-    for (int k = lane; k < cr; k += 32) dst[k] = src ? __ldg(src + from[k]) : from[k];
+  const int staged = min(nf, Q.scap);
+  __syncwarp();
+  const short* theirs = stage + (t & ~31) * (kStageCap + 1);
+#pragma unroll 4
+  for (int rr = 0; rr < 32; ++rr) {
+    const int cr = __shfl_sync(0xffffffffu, staged, rr), to = __shfl_sync(0xffffffffu, row, rr);
+    int* dst = ids + (size_t)to * Q.max_nb;
+    const short* from = theirs + rr * (kStageCap + 1);
+    for (int k = lane; k < cr; k += 32) {
+      const int d = from[k], j = i - lane + rr + d;
+      if (d) dst[k] = src ? __ldg(src + j) : j;
+    }
   }
 }
 
 // outside: the out-of-domain flag of the hashing of `pos` (NULL: unknown).
-int launch_grid_frnn(const GridView& G, int n, const float2* pos, const int* start, const int* count, float r,
-                     float Lx, float Ly, int max_nb, int* counts, int* ids, unsigned long long* ovf,
-                     const int* src, cudaStream_t s, const int* outside) {
+int launch_grid_frnn(const GridView& G, int n, const float2* pos, const int* start, float r, float Lx, float Ly,
+                     int max_nb, int* counts, int* ids, unsigned long long* ovf, const int* src, cudaStream_t s,
+                     const int* outside) {
   const unsigned blocks = (unsigned)((n + kFrnnThreads - 1) / kFrnnThreads);
   // the minimum image by row segment is exact when every candidate cell lies
   // within 0.45 of the domain of the query point (stencil half-width + a
@@ -881,12 +947,9 @@ int launch_grid_frnn(const GridView& G, int n, const float2* pos, const int* sta
     return cells >= 20 && (1.0001 * r + margin + c) * 1.01 <= 0.45 * L;
   };
   const int by_segment = G.periodic && outside && fits(G.cx, Lx, G.nx, G.minx) && fits(G.cy, Ly, G.ny, G.miny);
-  if (G.periodic)
-    k_grid_frnn<true><<<blocks, kFrnnThreads, 0, s>>>(G, n, pos, start, count, r, Lx, Ly, max_nb, counts, ids, ovf, src,
-                                                      outside, by_segment);
-  else
-    k_grid_frnn<false><<<blocks, kFrnnThreads, 0, s>>>(G, n, pos, start, count, r, Lx, Ly, max_nb, counts, ids, ovf,
-                                                       src, outside, 0);
+  const NearQuery Q = {r, 1.0f / G.cx, 1.0f / G.cy, Lx, Ly, max_nb, std::min(max_nb, kStageCap)};
+  auto kernel = G.periodic ? k_grid_frnn<true> : k_grid_frnn<false>;
+  kernel<<<blocks, kFrnnThreads, 0, s>>>(G, Q, n, pos, start, counts, ids, ovf, src, outside, by_segment);
   QCK(cudaGetLastError());
   return MCL_OK;
 }
@@ -1225,7 +1288,7 @@ int mcl_grid_frnn_ids(mcl_grid* g, float r, int max_nb, int32_t* counts, int32_t
   const GridView G = view_of(g);
   unsigned long long* ovf = (unsigned long long*)g->scan_tmp;
   QCK(cudaMemsetAsync(ovf, 0, 8, s));
-  const int rc = launch_grid_frnn(G, n, g->tmp, g->start, g->count, r, g->cx * g->nx, g->cy * g->ny, max_nb, counts,
+  const int rc = launch_grid_frnn(G, n, g->tmp, g->start, r, g->cx * g->nx, g->cy * g->ny, max_nb, counts,
                                   ids, ovf, g->src, s, g->count + g->ncells);
   if (rc != MCL_OK) return rc;
   if (overflow) {
@@ -1267,7 +1330,7 @@ int mcl_grid_frnn(mcl_grid* g, const mcl_float2* pos, float r, int max_nb, int32
   const GridView G = view_of(g);
   unsigned long long* ovf = (unsigned long long*)g->scan_tmp;
   QCK(cudaMemsetAsync(ovf, 0, 8, s));
-  const int rc = launch_grid_frnn(G, n, (const float2*)pos, g->start, g->count, r, g->cx * g->nx, g->cy * g->ny,
+  const int rc = launch_grid_frnn(G, n, (const float2*)pos, g->start, r, g->cx * g->nx, g->cy * g->ny,
                                   max_nb, counts, ids, ovf, nullptr, s, nullptr);
   if (rc != MCL_OK) return rc;
   if (overflow) {
@@ -1330,30 +1393,30 @@ __global__ void k_bgrid_hash(int V, const float2* pos, const unsigned char* vfix
 // mesh); disk-culled rows of the mesh's grid, branch-free candidate test,
 // ids staged per thread in shared memory, sorted there and written out one row
 // per warp step.  Rows: out[v*F] = count, out[v*F + 1 + k] ascending.
+// The stage rows are as long as the caller's.  Bound by the candidates' loads and the
+// sort (r = 2 x spacing, 1,400,000 points, 12.6 neighbours: 201 -> 154 us).
 constexpr int kBStage = 48;
 
-__global__ void __launch_bounds__(kFrnnThreads) k_bgrid_frnn(int n, const float2* __restrict__ spos,
+__global__ void __launch_bounds__(kFrnnThreads, kFrnnBlocks) k_bgrid_frnn(int n, const float2* __restrict__ spos,
                                                             const int* __restrict__ src, const int* __restrict__ vcomp,
                                                             const int4* __restrict__ par, const float* __restrict__ rc,
-                                                            float lo, const int* __restrict__ start,
-                                                            const int* __restrict__ count, int F, int* __restrict__ out,
-                                                            unsigned long long* overflow) {
-  __shared__ int stage[kFrnnThreads * (kBStage + 1)];
-  __shared__ int cnts[kFrnnThreads];
-  __shared__ int rows[kFrnnThreads];
-  const int t = threadIdx.x, row0 = blockIdx.x * kFrnnThreads, i = row0 + t;
-  int* mine = stage + t * (kBStage + 1);
-  const int cap = F - 1;  // <= kBStage (checked by the host)
-  int nf = 0;
+                                                            float lo, const int* __restrict__ start, int F,
+                                                            int* __restrict__ out, unsigned long long* overflow) {
+  extern __shared__ int bstage[];
+  const int t = threadIdx.x, lane = t & 31, i = blockIdx.x * kFrnnThreads + t;
+  const int cap = F - 1;        // <= kBStage (checked by the host)
+  const int len = F | 1;        // one more than cap, and odd
+  int* mine = bstage + t * len;
+  int nf = 0, v = 0;
   if (i < n) {
-    const int v = __ldg(src + i);
-    rows[t] = v;
+    v = __ldg(src + i);
     const int mesh = vcomp ? __ldg(vcomp + v) : 0;
     const int4 q = __ldg(par + mesh);
     const float c = __int_as_float(q.x), inv = 1.0f / c;
     const float r = __ldg(rc + mesh);
     const float r2 = __fmul_rn(r, r);
     const float2 p = spos[i];
+    const unsigned long long minus_p = pair_of(-p.x, -p.y);
     const int nx = q.y;
     const float mg = 1e-3f * c + 1e-5f * (fabsf(p.x) + fabsf(p.y) + fabsf(lo) + r);
     const float px = p.x - lo, py = p.y - lo;
@@ -1366,28 +1429,24 @@ __global__ void __launch_bounds__(kFrnnThreads) k_bgrid_frnn(int n, const float2
       if (yy == 0) slo = -INFINITY;
       if (yy == nx - 1) shi = INFINITY;
       const float dym = fmaxf(fmaxf(slo - py, py - shi) - mg, 0.f);
-      const float hw = sqrtf(fmaxf(r2 - dym * dym, 0.f)) * 1.0001f + mg;
+      const float hw = near_sqrt(fmaxf(r2 - dym * dym, 0.f)) * 1.0001f + mg;
       int xlo = (int)floorf(fmaxf(fminf((px - hw) * inv, 1e9f), -1e9f));
       int xhi = (int)floorf(fmaxf(fminf((px + hw) * inv, 1e9f), -1e9f));
       xlo = xlo < 0 ? 0 : (xlo >= nx ? nx - 1 : xlo);
       xhi = xhi < 0 ? 0 : (xhi >= nx ? nx - 1 : xhi);
-      const int base = q.z + yy * nx;
-      const int b = __ldg(start + base + xlo);
-      const int e = __ldg(start + base + xhi) + __ldg(count + base + xhi);
+      const int* row = start + q.z + yy * nx;
+      const int b = __ldg(row + xlo), e = __ldg(row + xhi + 1);
+      const unsigned long long* at = reinterpret_cast<const unsigned long long*>(spos);
       if (nf + (e - b) <= cap) {
 #pragma unroll 4
         for (int j = b; j < e; ++j) {
-          const float2 o = spos[j];
-          const float dx = __fsub_rn(p.x, o.x), dy = __fsub_rn(p.y, o.y);
-          const bool hit = (__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= r2) & (j != i);
+          const bool hit = (pair_norm2(pair_add(at[j], minus_p)) <= r2) & (j != i);
           mine[nf] = j;
           nf += hit ? 1 : 0;
         }
       } else {
         for (int j = b; j < e; ++j) {
-          const float2 o = spos[j];
-          const float dx = __fsub_rn(p.x, o.x), dy = __fsub_rn(p.y, o.y);
-          if ((__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)) <= r2) & (j != i)) {
+          if ((pair_norm2(pair_add(at[j], minus_p)) <= r2) & (j != i)) {
             if (nf < cap) mine[nf] = j;
             ++nf;
           }
@@ -1405,15 +1464,17 @@ __global__ void __launch_bounds__(kFrnnThreads) k_bgrid_frnn(int n, const float2
       mine[bb + 1] = x;
     }
     nf = m;
+  } else {
+    nf = -1;
   }
-  cnts[t] = i < n ? nf : -1;
-  __syncthreads();
-  const int lane = t & 31;
-  for (int rr = t >> 5; rr < kFrnnThreads && row0 + rr < n; rr += kFrnnThreads / 32) {
-    const int cr = cnts[rr];
-    int* dst = out + (size_t)rows[rr] * F;
-    const int* from = stage + rr * (kBStage + 1);
-    if (lane == 0) dst[0] = cr;
+  __syncwarp();
+  const int* theirs = bstage + (t & ~31) * len;
+#pragma unroll 4
+  for (int rr = 0; rr < 32; ++rr) {
+    const int cr = __shfl_sync(0xffffffffu, nf, rr), to = __shfl_sync(0xffffffffu, v, rr);
+    int* dst = out + (size_t)to * F;
+    const int* from = theirs + rr * len;
+    if (lane == 0 && cr >= 0) dst[0] = cr;
     for (int k = lane; k < cr; k += 32) dst[k + 1] = from[k];
   }
 }
@@ -1483,8 +1544,9 @@ extern "C" int mcl_batch_frnn_grid(mcl_mesh* m, const float* r_host, const float
                m->bg_bucket, pos, nullptr, m->bg_start, nullptr, m->bg_src, m->bg_pos, nullptr, s);
   unsigned long long* ovf = m->scratch + 4;
   QCK(cudaMemsetAsync(ovf, 0, 8, s));
-  k_bgrid_frnn<<<(unsigned)((npts + kFrnnThreads - 1) / kFrnnThreads), kFrnnThreads, 0, s>>>(
-      npts, m->bg_pos, m->bg_src, m->vcomp, m->bg_par, r_dev, lo, m->bg_start, m->bg_count, max_frnn, out_dev, ovf);
+  k_bgrid_frnn<<<(unsigned)((npts + kFrnnThreads - 1) / kFrnnThreads), kFrnnThreads,
+                 sizeof(int) * kFrnnThreads * (max_frnn | 1), s>>>(npts, m->bg_pos, m->bg_src, m->vcomp, m->bg_par,
+                                                                   r_dev, lo, m->bg_start, max_frnn, out_dev, ovf);
   QCK(cudaGetLastError());
   if (overflow) {
     unsigned long long t = 0;
@@ -1569,7 +1631,7 @@ extern "C" int mcl_grid_frnn_noalloc(const mcl_float2* pos, int64_t n, float min
   k_grid_hash<<<(nn + 255) / 256, 256, 0, s>>>(G, nn, (const float2*)pos, cell, count, perm, nullptr);
   launch_cells(nn, nn, ncells, cell, count, ticket, perm, local, pre, bucket, (const float2*)pos, nullptr, start, perm,
                src, (float2*)sorted_pos, nullptr, s);
-  const int rc2 = launch_grid_frnn(G, nn, (const float2*)sorted_pos, start, count, r, cell_x * cells_x,
+  const int rc2 = launch_grid_frnn(G, nn, (const float2*)sorted_pos, start, r, cell_x * cells_x,
                                    cell_y * cells_y, max_nb, counts, ids, ovf, nullptr, s, nullptr);
   if (rc2 != MCL_OK) return rc2;
   if (overflow) {

@@ -59,3 +59,46 @@ def test_tables(M, n, nx, ny, crowd, periodic):
     assert np.array_equal(pos.cpu().numpy(), p[order])
     assert np.array_equal(vel.cpu().numpy(), v[order])
     g.close()
+
+
+@pytest.mark.parametrize("periodic", [False, True])
+def test_neighbours_far_apart_in_the_order(M, periodic):
+    """More points than 16 bits count: rows met across the wrap, and one cell so
+    crowded that its own points are that far apart."""
+    import torch
+    from scipy.spatial import cKDTree
+
+    n, L, r, F = 90000, 300.0, np.float32(2.25), 32
+    rng = np.random.default_rng(7)
+    p = (rng.random((n, 2)) * L).astype(np.float32)
+    g = M.GridCount2d(n, (0.0, 0.0), (1.5, 1.5), (200, 200), periodic=periodic)
+    counts = torch.zeros(n, dtype=torch.int32, device="cuda")
+    ids = torch.full((n, F), -1, dtype=torch.int32, device="cuda")
+    g.build(torch.from_numpy(p).cuda())
+    g.frnn_ids(float(r), F, counts, ids)
+    got_c, got = counts.cpu().numpy(), ids.cpu().numpy()
+    tree = cKDTree(p.astype(np.float64), boxsize=L if periodic else None)
+    for i in np.concatenate([np.arange(40), rng.integers(0, n, 400), np.argsort(p[:, 1])[:200]]):
+        near = np.array(sorted(set(tree.query_ball_point(p[i].astype(np.float64), float(r) + 0.01)) - {i}))
+        d = (p[i] - p[near]).astype(np.float32)
+        if periodic:
+            d = np.where(np.abs(d) > np.float32(L / 2), (d - np.copysign(np.float32(L), d)).astype(np.float32), d)
+        want = near[(d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]).astype(np.float32) <= r * r]
+        assert got_c[i] == len(want)
+        assert np.array_equal(np.sort(got[i, :got_c[i]]), want)
+        assert (got[i, got_c[i]:] == -1).all()
+    g.close()
+
+    k = 40000
+    p = np.full((k, 2), 10.0, np.float32)
+    g = M.GridCount2d(k, (0.0, 0.0), (1.5, 1.5), (200, 200), periodic=periodic)
+    counts = torch.zeros(k, dtype=torch.int32, device="cuda")
+    ids = torch.full((k, 60), -1, dtype=torch.int32, device="cuda")
+    g.build(torch.from_numpy(p).cuda())
+    assert g.frnn_ids(1.0, 60, counts, ids) == k
+    got = ids.cpu().numpy()
+    assert (counts.cpu().numpy() == 60).all()
+    for i in (0, 1, 47, 59, 60, 61, 32767, 32768, 32830, k - 1):
+        want = np.arange(61)
+        assert np.array_equal(got[i], want[want != i][:60])
+    g.close()
