@@ -1795,9 +1795,9 @@ __device__ bool phase_insert(cg::grid_group& g, const KParams& P, unsigned& stam
 // End of a launch: publish this launch's counters and status for the host,
 // add them to the running totals, and leave the working state clean for the
 // next launch (so no reset launch or memset precedes the next step).
-// The step counters of the last launch in the public record layout.
-__device__ void publish_stats(const DevState* st, mcl_step_stats* out) {
-  const unsigned long long* c = st->last;
+// The step counters c of a launch in the public record layout.
+__device__ __forceinline__ void publish_counts(const unsigned long long (&c)[C_COUNT], int status, int site,
+                                               mcl_step_stats* out) {
   out->inverted_faces = (int64_t)c[C_INVERTED];
   out->reverted_vertices = (int64_t)c[C_REVERTED];
   out->removed_vertices = (int64_t)c[C_REMOVED];
@@ -1811,32 +1811,48 @@ __device__ void publish_stats(const DevState* st, mcl_step_stats* out) {
   out->orient_fp64 = (int64_t)c[C_ORIENT_FP64];
   out->orient_exact = (int64_t)c[C_ORIENT_EXACT];
   out->sos_decisions = (int64_t)c[C_SOS];
-  out->status = st->last_status;
-  out->error_site = st->last_site;
-  out->failed_launches = st->last_status != MCL_OK ? 1 : 0;
+  out->status = status;
+  out->error_site = site;
+  out->failed_launches = status != MCL_OK ? 1 : 0;
   out->substep_vertices = (int64_t)c[C_SUBSTEP_DONE];
 }
 
+// By one warp, a counter per lane: a lone thread's reads and writes, each waiting for
+// the last, and the copy of the record that followed closed a step with 6 us more.
 __device__ void finish_launch(const KParams& P, unsigned stamp) {
+  static_assert(C_COUNT <= 32, "a lane per counter");
   DevState* st = P.st;
+  const int lane = threadIdx.x & 31;
   // L2-coherent reads: other blocks' atomics and stores are not in this SM's L1
-  for (int i = 0; i < C_COUNT; ++i) {
-    const unsigned long long c = __ldcg(&st->c[i]);
-    st->last[i] = c;
-    st->tot[i] += c;
-    st->c[i] = 0;
+  unsigned long long c = 0, tot = 0;
+  if (lane < C_COUNT) {
+    c = __ldcg(&st->c[lane]);
+    tot = __ldcg(&st->tot[lane]);
   }
-  const int status = __ldcg(&st->status);
-  st->calls += 1;
-  if (status != MCL_OK) st->failed += 1;
-  const bool repaired = st->last[C_INVERTED] != 0;
-  for (int i = 0; i < 4; ++i) {
-    if (!repaired) st->ts[43 + i] = __ldcg(&st->tsmax[i]);
-    st->tsmax[i] = 0;
+  const unsigned long long tm = __ldcg(&st->tsmax[lane & 3]);
+  const int status = __ldcg(&st->status), site = __ldcg(&st->site), movers = __ldcg(&st->movers_now);
+  const unsigned long long calls = __ldcg(&st->calls), failed = __ldcg(&st->failed);
+  if (lane < C_COUNT) {
+    st->last[lane] = c;
+    st->tot[lane] = tot + c;
+    st->c[lane] = 0;
   }
+  const bool repaired = __shfl_sync(kFull, c, C_INVERTED) != 0;
+  if (lane < 4) {
+    if (!repaired) st->ts[43 + lane] = tm;
+    st->tsmax[lane] = 0;
+  }
+  if (P.stats_out) {  // host-mapped: no copy launch
+    unsigned long long all[C_COUNT];
+#pragma unroll
+    for (int i = 0; i < C_COUNT; ++i) all[i] = __shfl_sync(kFull, c, i);
+    if (lane == 0) publish_counts(all, status, site, P.stats_out);
+  }
+  if (lane != 0) return;
+  st->calls = calls + 1;
+  if (status != MCL_OK) st->failed = failed + 1;
   st->last_status = status;
-  st->last_site = __ldcg(&st->site);
-  if (P.stats_out) publish_stats(st, P.stats_out);  // host-mapped: no copy launch
+  st->last_site = site;
   st->status = 0;
   st->site = 0;
   st->wl_count[0] = st->wl_count[1] = 0;
@@ -1849,7 +1865,7 @@ __device__ void finish_launch(const KParams& P, unsigned stamp) {
   st->star_made = 0;
   st->fix_all = 0;
   st->mark_ovf = 0;
-  st->movers_last = __ldcg(&st->movers_now);
+  st->movers_last = movers;
   st->movers_now = 0;
   st->epoch = stamp;
 }
@@ -2970,17 +2986,23 @@ __global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KP
   // threads' counter updates before thread 0's fence, and the fence (which is
   // cumulative) orders them before the block's arrival.
   __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicMax(&P.st->stamp_max, stamp);
-    __threadfence();
-    if (atomicAdd(&P.st->arrived, 1u) == gridDim.x - 1) {
+  if (threadIdx.x < 32) {
+    int last = 0;
+    if (threadIdx.x == 0) {
+      atomicMax(&P.st->stamp_max, stamp);
       __threadfence();
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      P.st->ts[kTimeline - 1] = t;
+      last = atomicAdd(&P.st->arrived, 1u) == gridDim.x - 1 ? 1 : 0;
+    }
+    if (__shfl_sync(kFull, last, 0)) {
+      __threadfence();
       finish_launch(P, __ldcg(&P.st->stamp_max));
-      P.st->arrived = 0;
-      P.st->stamp_max = 0;
+      if (threadIdx.x == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        P.st->ts[kTimeline - 1] = t;
+        P.st->arrived = 0;
+        P.st->stamp_max = 0;
+      }
     }
   }
 }
@@ -3186,7 +3208,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_build(const __grid_constant__ K
   }
   flush_counters(P, lc);
   g.sync();
-  if (gtid == 0) finish_launch(P, stamp);
+  if (gtid < 32) finish_launch(P, stamp);
 }
 
 // ---------------------------------------------------------------------------
@@ -3308,15 +3330,20 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   cudaError_t e = cudaMalloc((void**)&m->slab, at);
   if (e == cudaSuccess)
     for (const auto& [p, off] : parts) *p = m->slab + off;
-  // the mirror of the device state, and behind it the counts that queries write: pages
-  // of the host's, pinned in place
+  // the mirror of the device state, behind it the counts that queries write and a step's
+  // record: pages of the host's, pinned in place
   if (e == cudaSuccess) {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE), bytes = (sizeof(DevState) + 64 + page - 1) / page * page;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), bytes = (sizeof(DevState) + 64 + sizeof(mcl_step_stats) + page - 1) / page * page;
     m->st_host = static_cast<DevState*>(std::aligned_alloc(page, bytes));
     e = m->st_host ? cudaHostRegister(m->st_host, bytes, cudaHostRegisterMapped) : cudaErrorMemoryAllocation;
   }
   if (e == cudaSuccess) m->counts_host = reinterpret_cast<unsigned long long*>(m->st_host + 1);
   if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&m->counts_dev, m->counts_host, 0);
+  static_assert(sizeof(DevState) % 8 == 0, "what follows the state in the mirror's pages");
+  if (e == cudaSuccess) {
+    m->stats_host = reinterpret_cast<mcl_step_stats*>(m->counts_host + 8);
+    m->stats_map = reinterpret_cast<mcl_step_stats*>(m->counts_dev + 8);
+  }
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     free_mesh(m);
@@ -3576,16 +3603,16 @@ static void fill_stats_from(const unsigned long long* c, int status, int site, m
   o->failed_launches = 0;
 }
 
+static int checked(mcl_mesh* m, int status) {
+  m->last_status = status;
+  return status == MCL_OK ? MCL_OK : fail(status, std::string("device status: ") + mcl_status_string(status));
+}
 static int finish(mcl_mesh* m, cudaStream_t s, mcl_step_stats* stats) {
   if (!stats) return MCL_OK;
   CK(cudaMemcpyAsync(m->st_host, m->st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   fill_stats(*m->st_host, stats);
-  m->last_status = m->st_host->last_status;
-  if (m->st_host->last_status != MCL_OK)
-    return fail(m->st_host->last_status,
-                std::string("device status: ") + mcl_status_string(m->st_host->last_status));
-  return MCL_OK;
+  return checked(m, m->st_host->last_status);
 }
 
 // Run the engine.  Position buffers: pos[cur] holds the positions the mesh
@@ -3597,7 +3624,7 @@ static int finish(mcl_mesh* m, cudaStream_t s, mcl_step_stats* stats) {
 static int run_step(mcl_mesh* m, int move_mode, const float2* d, cudaStream_t s, mcl_step_stats* stats,
                     mcl_step_stats* stats_mapped = nullptr) {
   KParams P = make_params(m, ENGINE_STEP);
-  P.stats_out = stats_mapped;
+  P.stats_out = stats ? m->stats_map : stats_mapped;  // no caller gives both
   if (move_mode != MOVE_NONE) {
     if (m->dirty) {
       // the launch writes the other position buffer for the active meshes
@@ -3639,7 +3666,10 @@ static int run_step(mcl_mesh* m, int move_mode, const float2* d, cudaStream_t s,
   if (rc != MCL_OK) return rc;
   m->valid_cur = true;
   m->delaunay = true;  // a step ends Delaunay (or with an error status)
-  return finish(m, s, stats);
+  if (!stats) return MCL_OK;
+  CK(cudaStreamSynchronize(s));
+  *stats = *m->stats_host;
+  return checked(m, stats->status);
 }
 
 // Structural invariants of the device mesh (counted per kind):
@@ -3913,7 +3943,10 @@ int mcl_step_host(mcl_mesh* m, const mcl_float2* d_host, void* stream, mcl_step_
 namespace mcl {
 // the counters of the last launch as an mcl_step_stats, in device memory
 __global__ void k_publish_stats(const DevState* st, mcl_step_stats* out) {
-  if (threadIdx.x == 0) publish_stats(st, out);
+  if (threadIdx.x != 0) return;
+  unsigned long long c[C_COUNT];
+  for (int i = 0; i < C_COUNT; ++i) c[i] = st->last[i];
+  publish_counts(c, st->last_status, st->last_site, out);
 }
 }  // namespace mcl
 

@@ -381,6 +381,8 @@ struct mcl_mesh {
   unsigned long long* scratch;  // small device scratch for query counters (kScratchBytes)
   unsigned long long* counts_host;  // behind st_host: counts of the last counted queries
   unsigned long long* counts_dev;   // the same, as the device sees them
+  mcl_step_stats* stats_host;       // behind those: the record a step writes when its caller waits for it
+  mcl_step_stats* stats_map;        // ... as the device sees it
   mcl::DevState* st;
   mcl::DevState* st_host;  // pinned mirror (own pages, registered)
   int coop_blocks;         // k_step grid
