@@ -393,6 +393,7 @@ struct mcl_mesh {
   int nsm;                 // SMs of the device
   int max_blocks_per_sm;   // k_step occupancy limit
   int tail_items;          // single-block flip-round threshold
+  bool tail_auto;          // ... not set by the caller: at most one edge per thread
   int rm_tile;             // removal tile (mcl_mesh_set_removal_tile; 0 = automatic)
   int substeps;            // repair sub-steps before removal (mcl_mesh_set_substeps)
   bool delaunay;           // the last launch left the mesh Delaunay (set when a step or build is launched)
