@@ -195,6 +195,7 @@ struct PView {
   int* wl0;                   // edge work-lists: the edges whose quads a round's flips changed
   int* wl1;
   unsigned* qstamp;           // the round an edge was last queued for
+  int* vhe;                   // an outgoing half-edge per vertex, kept by the flips (NULL: none is)
 };
 
 MCL_HD void p_add(unsigned long long* p, unsigned long long v) {
@@ -536,6 +537,12 @@ MCL_HD void p_body_flip(const PView& V, int e, unsigned stamp, int next) {
   const int a = q.x, b = q.y, c = q.z, d = q.w;
   const int n0 = w.x, p0 = w.y, n1 = w.z, p1 = w.w;
   const int h0 = 2 * e, h1 = 2 * e + 1;
+  if (V.vhe) {
+    // only e's own flip takes 2 e and 2 e + 1 away from a and b
+    const int va = V.vhe[a], vb = V.vhe[b];
+    if (va == h0) V.vhe[a] = n1;
+    if (vb == h1) V.vhe[b] = n0;
+  }
   V.ev[e] = PI4{d, c, a, b};
   V.en[e] = PI4{p0, n1, p1, n0};
   V.eo[e] = f.eo;
@@ -1173,8 +1180,23 @@ MCL_HD long long p_ring_key(int id, unsigned off) { return ((long long)id << 8) 
 // at most max_ring - 1 of them; slot 0 holds the count (the reference's ring
 // layout, include/kernels.cuh:54-84).  offs (may be null) receives, in the same
 // layout, each neighbour's copy offset relative to v (an offset byte).
-MCL_HD void p_body_ring(const PView& V, const int* vhe, int v, bool column, int max_ring, int* ring,
-                        unsigned char* offs) {
+// The star is walked once, both ways at a time (a spoke's record gives the next one on
+// either side), its neighbours kept in the stage S and written from the smallest on;
+// stars wider than the stage are walked again.
+struct PRingLocal {
+  int id_[16];
+  unsigned char off_[16];
+  MCL_HD int cap() const { return 16; }
+  MCL_HD int id(int i) const { return id_[i]; }
+  MCL_HD unsigned off(int i) const { return off_[i]; }
+  MCL_HD void set(int i, int id, unsigned off) {
+    id_[i] = id;
+    off_[i] = (unsigned char)off;
+  }
+};
+template <typename Stage>
+MCL_HD void p_ring_row(const PView& V, const int* vhe, int v, bool column, int max_ring, int* ring,
+                       unsigned char* offs, Stage& S) {
   const int h0 = vhe[v];
   const unsigned H = 2u * (unsigned)V.E;
   if ((unsigned)h0 >= H || p_origin(V, h0) != v) {
@@ -1184,8 +1206,91 @@ MCL_HD void p_body_ring(const PView& V, const int* vhe, int v, bool column, int 
   const size_t stride = column ? (size_t)V.n : 1;
   int* row = column ? ring + v : ring + (size_t)v * max_ring;
   unsigned char* orow = offs ? (column ? offs + v : offs + (size_t)v * max_ring) : nullptr;
-  int start = h0, deg = 0, h = h0;
+  const int cap = max_ring - 1, room = S.cap();
+  // clockwise neighbours from slot 0 up, counter-clockwise ones from the last slot down
+  int fw = 0, bw = 0, best_at = 0;
   long long best = 0;
+  auto put = [&](int slot, int id, Off o) {
+    const unsigned ob = off_byte(o);
+    S.set(slot, id, ob);
+    const long long key = p_ring_key(id, ob);
+    if (fw + bw == 0 || key < best) {
+      best = key;
+      best_at = slot;
+    }
+  };
+  // a spoke's record also names the neighbours beside it, so every other one is read
+  int id_f, id_b;
+  Off off_f, off_b;
+  bool known = true;  // (id_f, off_f) and (id_b, off_b) are the next spokes' ends
+  {
+    const PI4 q = V.ev[h0 >> 1];
+    const unsigned o = V.eo[h0 >> 1];
+    const int side = h0 & 1;
+    put(0, side ? q.x : q.y, eo_target(o, side));
+    fw = 1;
+    id_f = side ? q.z : q.w;
+    off_f = off_add(eo_target(o, side), eo_apex(o, side ^ 1));
+    id_b = side ? q.w : q.z;
+    off_b = eo_apex(o, side);
+  }
+  int f = h0, b = h0;
+  bool closed = false;
+  while (fw + bw <= room) {
+    const PI4 wf = V.en[f >> 1], wb = V.en[b >> 1];
+    const int nf = (f & 1) ? wf.x : wf.z;        // next(twin(f))
+    const int pb = ((b & 1) ? wb.w : wb.y) ^ 1;  // twin(prev(b))
+    if ((unsigned)nf >= H || (unsigned)pb >= H) {
+      p_error(V, MCL_ERR_DEGENERATE_INPUT, 8);
+      return;
+    }
+    closed = nf == b;
+    if (closed || fw + bw == room) break;
+    PI4 qf, qb;
+    unsigned of = 0, ob = 0;
+    if (!known) {
+      qf = V.ev[nf >> 1];
+      of = V.eo[nf >> 1];
+      qb = V.ev[pb >> 1];
+      ob = V.eo[pb >> 1];
+      id_f = (nf & 1) ? qf.x : qf.y;
+      off_f = eo_target(of, nf & 1);
+      id_b = (pb & 1) ? qb.x : qb.y;
+      off_b = eo_target(ob, pb & 1);
+    }
+    put(fw, id_f, off_f);
+    ++fw;
+    closed = nf == pb;
+    if (closed || fw + bw == room) break;
+    put(room - 1 - bw, id_b, off_b);
+    ++bw;
+    if (!known) {
+      id_f = (nf & 1) ? qf.z : qf.w;
+      off_f = off_add(off_f, eo_apex(of, (nf & 1) ^ 1));
+      id_b = (pb & 1) ? qb.w : qb.z;
+      off_b = eo_apex(ob, pb & 1);
+    }
+    known = !known;
+    f = nf;
+    b = pb;
+  }
+  if (closed) {
+    const int deg = fw + bw, cnt = deg < cap ? deg : cap;
+    int at = best_at;
+    for (int k = 0; k < cnt; ++k) {
+      row[(size_t)(k + 1) * stride] = S.id(at);
+      if (orow) orow[(size_t)(k + 1) * stride] = (unsigned char)S.off(at);
+      // clockwise: the front's slots, then from the back's last in to its first
+      ++at;
+      if (at == fw) at = room - bw;
+      if (at == room) at = 0;
+    }
+    row[0] = cnt;
+    if (orow) orow[0] = 0;
+    if (deg > cap) p_add(&V.cnt->truncated, 1);
+    return;
+  }
+  int start = h0, deg = 0, h = h0;
   do {
     const int nb = p_origin(V, h ^ 1);
     const unsigned ob = off_byte(eo_target(V.eo[h >> 1], h & 1));
@@ -1205,7 +1310,6 @@ MCL_HD void p_body_ring(const PView& V, const int* vhe, int v, bool column, int 
     p_error(V, MCL_ERR_DEGENERATE_INPUT, 9);
     return;
   }
-  const int cap = max_ring - 1;
   const int cnt = deg < cap ? deg : cap;
   h = start;
   for (int k = 0; k < cnt; ++k) {
@@ -1216,6 +1320,11 @@ MCL_HD void p_body_ring(const PView& V, const int* vhe, int v, bool column, int 
   row[0] = cnt;
   if (orow) orow[0] = 0;
   if (deg > cap) p_add(&V.cnt->truncated, 1);
+}
+MCL_HD void p_body_ring(const PView& V, const int* vhe, int v, bool column, int max_ring, int* ring,
+                        unsigned char* offs) {
+  PRingLocal S;
+  p_ring_row(V, vhe, v, column, max_ring, ring, offs, S);
 }
 
 // vertex v: the ring neighbour nearest to v on the torus (smallest id among
