@@ -562,7 +562,10 @@ __device__ bool phase_classify(cg::grid_group& g, const KParams& P, unsigned qst
           // first stamp: the queue mark is a plain store (no atomic waited for)
           __stcg(P.qmark + e[j], qstamp);
           mark_quad<kFixedPos>(P, r, qstamp);
-          claim_edge(P, e[j], sc);
+          // once a face has turned over no flip round uses these claims, so a thread
+          // that has seen one claims no more (1M random walkers: 85 -> 78 us)
+          if (!kFixedPos || bad == 0) claim_edge(P, e[j], sc);
+          else __stcg(P.cand + e[j], sc);
           mine[k++] = e[j];
         }
       }
