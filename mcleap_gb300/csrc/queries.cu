@@ -325,14 +325,16 @@ __device__ __noinline__ void frnn_serial(const MeshView M, int i, float r2, int 
   if (overflow && (over || nf > cap)) atomicAdd(overflow, 1ull);
 }
 
-// A warp's search, breadth first: two lanes walk the ring of one vertex of the
+// Half a warp's search, breadth first: two lanes walk the ring of one vertex of the
 // frontier from its first spoke, one each way, until they meet; a lane's neighbour
 // within r joins through a hash set in shared memory.  The search is a chain of
 // dependent loads, so the time is the number of steps one after another: about
 // four a level for a ring of six, three or four levels for r = 2 x spacing, where a
 // thread alone takes a step for each of some eighty spokes and looks each up in its
-// own list in local memory.  60,000 queries, r = 2 x spacing, GB300: 567 us by
-// threads, 168 us by warps.
+// own list in local memory.  With a warp to a query 13 of its lanes had work and it was
+// bound by instruction issue (2600 a query); a frontier is seldom wider than the eight
+// vertices that half a warp takes at once.  60,000 queries, r = 2 x spacing, GB300:
+// 567 us by threads, 168 us by warps; the served list 163 us by warps, 120 by half warps (127 by quarters).
 constexpr int kFrnnWarps = 4;
 constexpr int kFrnnFound = 64;
 constexpr int kFrnnHash = 128;
@@ -341,19 +343,23 @@ __device__ __forceinline__ int mv_prev(const MeshView& M, int h) {
   return __ldg(reinterpret_cast<const int*>(M.en) + 4 * (h >> 1) + 2 * (h & 1) + 1);
 }
 
-__device__ __forceinline__ bool warp_search(const MeshView& M, int i, float r2, int* found, int* hash, int* count) {
-  const int lane = threadIdx.x & 31, way = lane & 1;
-  const unsigned lt = (1u << lane) - 1u;
+// Both halves of a warp call it together; a half with no query has i = -1.  Returns
+// false in a half that found more than its list holds.
+constexpr int kFrnnLanes = 16;
+__device__ __forceinline__ bool half_search(const MeshView& M, int i, float r2, int* found, int* hash, int* count) {
+  const int lane = threadIdx.x & 31, sub = lane & (kFrnnLanes - 1), way = lane & 1;
+  const unsigned half = ((1u << kFrnnLanes) - 1u) << (lane - sub), lt = half & ((1u << lane) - 1u);
 #pragma unroll
-  for (int k = 0; k < kFrnnHash / 32; ++k) hash[32 * k + lane] = -1;
+  for (int k = 0; k < kFrnnHash / kFrnnLanes; ++k) hash[kFrnnLanes * k + sub] = -1;
   __syncwarp();
-  const float2 pi = M.pos[i];
+  bool live = i >= 0, fits = true;
+  const float2 pi = live ? M.pos[i] : make_float2(0.f, 0.f);
   int nf = 0, lo = -1;  // the frontier: i, then found[lo .. hi)
-  while (lo < nf) {
+  while (__any_sync(0xffffffffu, live && lo < nf)) {
     const int hi = lo < 0 ? 0 : nf;
-    for (int c = lo; c < hi; c += 16) {
-      const int j = c + (lane >> 1);
-      const int u = lo < 0 ? (j == lo ? i : -1) : (j < hi ? found[j] : -1);
+    for (int c = lo; __any_sync(0xffffffffu, live && c < hi); c += kFrnnLanes / 2) {
+      const int j = c + (sub >> 1);
+      const int u = !live || c >= hi ? -1 : (lo < 0 ? (j == lo ? i : -1) : (j < hi ? found[j] : -1));
       const int h0 = u >= 0 ? __ldg(M.vhe + u) : -1;
       bool on = h0 >= 0;
       int cur = h0;
@@ -378,13 +384,12 @@ __device__ __forceinline__ bool warp_search(const MeshView& M, int i, float r2, 
             k = (k + 1) & (kFrnnHash - 1);
           }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, fresh);
+        const unsigned m = __ballot_sync(0xffffffffu, fresh) & half;
         if (fresh) {
           const int at = nf + __popc(m & lt);
           if (at < kFrnnFound) found[at] = w;
         }
         nf += __popc(m);
-        if (nf > kFrnnFound) return false;
         const int ocur = __shfl_xor_sync(0xffffffffu, cur, 1), onxt = __shfl_xor_sync(0xffffffffu, nxt, 1);
         if (on) {
           if (last || nxt == ocur || nxt < 0) on = false;  // met, or the one between has been taken
@@ -394,16 +399,17 @@ __device__ __forceinline__ bool warp_search(const MeshView& M, int i, float r2, 
           }
           cur = nxt;
         }
+        if (nf > kFrnnFound) on = live = fits = false;
       }
       __syncwarp();
     }
     lo = hi;
   }
   *count = nf;
-  return true;
+  return fits;
 }
 
-// Rows for the vertices verts[0 .. n) (NULL: all of them), a warp each.  With
+// Rows for the vertices verts[0 .. n) (NULL: all of them), half a warp each.  With
 // rcomp the radius of vertex i is rcomp[vcomp[i]] (one radius per mesh of a batch; a
 // plain mesh has vcomp == nullptr and one radius).
 __global__ void __launch_bounds__(32 * kFrnnWarps) k_mesh_frnn(MeshView M, const int* verts, int n, float r2,
@@ -411,40 +417,38 @@ __global__ void __launch_bounds__(32 * kFrnnWarps) k_mesh_frnn(MeshView M, const
                                                                unsigned long long* overflow,
                                                                unsigned long long* host, const float* rcomp,
                                                                const int* vcomp) {
-  __shared__ int found_s[kFrnnWarps][kFrnnFound];
-  __shared__ int hash_s[kFrnnWarps][kFrnnHash];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int q = blockIdx.x * kFrnnWarps + warp;
-  if (q < n) {
-    const int i = verts ? __ldg(verts + q) : q;
-    const int cap = max_frnn - 1;
-    int* row = layout == MCL_LAYOUT_COLUMN ? out + q : out + (size_t)q * max_frnn;
-    const size_t stride = layout == MCL_LAYOUT_COLUMN ? (size_t)n : 1;
-    if (i < 0 || i >= M.V || __ldg(M.vhe + i) < 0) {
-      if (lane == 0) row[0] = 0;
-    } else {
-      if (rcomp) {
-        const float rc = rcomp[vcomp ? vcomp[i] : 0];
-        r2 = __fmul_rn(rc, rc);
-      }
-      int* found = found_s[warp];
-      int nf = 0;
-      if (warp_search(M, i, r2, found, hash_s[warp], &nf)) {
-        __syncwarp();
-        for (int k = lane; k < nf; k += 32) {
-          const int x = found[k];
-          int rank = 0;
-          for (int j = 0; j < nf; ++j) rank += found[j] < x ? 1 : 0;
-          if (rank < cap) row[(size_t)(rank + 1) * stride] = x;
-        }
-        if (lane == 0) {
-          row[0] = nf < cap ? nf : cap;
-          if (overflow && nf > cap) atomicAdd(overflow, 1ull);
-        }
-      } else if (lane == 0) {
-        frnn_serial(M, i, r2, cap, stride, row, overflow);
-      }
+  constexpr int kPer = 32 / kFrnnLanes * kFrnnWarps;  // queries per block
+  __shared__ int found_s[kPer][kFrnnFound];
+  __shared__ int hash_s[kPer][kFrnnHash];
+  const int sub = threadIdx.x & (kFrnnLanes - 1), slot = threadIdx.x / kFrnnLanes;
+  const int q = blockIdx.x * kPer + slot;
+  int i = q < n ? (verts ? __ldg(verts + q) : q) : -1;
+  const int cap = max_frnn - 1;
+  int* row = layout == MCL_LAYOUT_COLUMN ? out + q : out + (size_t)q * max_frnn;
+  const size_t stride = layout == MCL_LAYOUT_COLUMN ? (size_t)n : 1;
+  if (i >= M.V || (i >= 0 && __ldg(M.vhe + i) < 0)) i = -1;
+  if (q < n && i < 0 && sub == 0) row[0] = 0;
+  if (rcomp && i >= 0) {
+    const float rc = rcomp[vcomp ? vcomp[i] : 0];
+    r2 = __fmul_rn(rc, rc);
+  }
+  const int* found = found_s[slot];
+  int nf = 0;
+  const bool fits = half_search(M, i, r2, found_s[slot], hash_s[slot], &nf);
+  __syncwarp();
+  if (i >= 0 && fits) {
+    for (int k = sub; k < nf; k += kFrnnLanes) {
+      const int x = found[k];
+      int rank = 0;
+      for (int j = 0; j < nf; ++j) rank += found[j] < x ? 1 : 0;
+      if (rank < cap) row[(size_t)(rank + 1) * stride] = x;
     }
+    if (sub == 0) {
+      row[0] = nf < cap ? nf : cap;
+      if (overflow && nf > cap) atomicAdd(overflow, 1ull);
+    }
+  } else if (i >= 0 && sub == 0) {
+    frnn_serial(M, i, r2, cap, stride, row, overflow);
   }
   if (host) count_done(overflow, host);
 }
@@ -1092,7 +1096,8 @@ int launch_mesh_frnn(mcl_mesh* m, const int* verts, int64_t n, float r2, const f
     return MCL_OK;
   }
   unsigned long long* host = overflow ? m->counts_host + kHostFrnn : nullptr;
-  k_mesh_frnn<<<(unsigned)((n + kFrnnWarps - 1) / kFrnnWarps), 32 * kFrnnWarps, 0, s>>>(
+  constexpr int kPer = 32 / kFrnnLanes * kFrnnWarps;
+  k_mesh_frnn<<<(unsigned)((n + kPer - 1) / kPer), 32 * kFrnnWarps, 0, s>>>(
       mesh_view(m), verts, (int)n, r2, layout, max_frnn, out, host ? m->scratch + kCellFrnn : nullptr,
       host ? m->counts_dev + kHostFrnn : nullptr, rcomp, rcomp ? m->vcomp : nullptr);
   QCK(cudaGetLastError());
