@@ -7,8 +7,13 @@
 //   classify  every edge: orientation of both faces, incircle of the quad;
 //             non-Delaunay edges go to a work-list       [delonize / untangle checks,
 //                                                          include/Device_Triangulation.h:31-116]
-//   repair    only when a face is inverted (the reference's untangle,
+//   stars     only when a face is inverted (the reference's untangle,
 //             include/Device_Triangulation.h:422-495, handles only its B/C cases):
+//             every vertex works out its own Delaunay star, checks it against its
+//             neighbours' and makes it again until all agree, then the mesh is
+//             rewritten (star.cuh); nothing is flipped;
+//   repair    in its place where few vertices of a large mesh moved, on the largest
+//             meshes, where sub-steps are asked for, or where stars do not agree:
 //             (1) revert vertices of non-positive faces to their old positions
 //                 until every face is positive;
 //             (2) remove the reverted vertices (flip each to degree 3, merge);
@@ -22,7 +27,8 @@
 //             highest-priority candidate always flips (no livelock).
 //
 // Rounds are separated by grid-wide barriers; nothing returns to the host
-// between rounds.  The same insertion rounds build the initial triangulation.
+// between rounds.  Stars from the points' Morton order build the initial triangulation,
+// and where they fail the repair's insertion rounds do.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -2715,6 +2721,12 @@ __device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, 
 // path, whose cost goes with the movers; the stars' goes with the mesh.
 constexpr int kStarSparse = 200000;
 
+// So is every step of a mesh larger than this: the stars' time goes with the vertices
+// (1.0 us a thousand), the removal path's rounds wait less per vertex the more they
+// hold.  Uniform points, sigma = 0.1 x spacing, stars and removal in ms: 1M 1.23 and
+// 1.72, 2M 2.11 and 2.35, 3M 3.12 and 2.92, 4M 4.06 and 3.29, 8.5M 8.34 and 6.05.
+constexpr int kStarMost = 2500000;
+
 // The vertices of the block's run marked with cs, in order, onto a list.
 __device__ __forceinline__ void star_marked(const KParams& P, unsigned cs, int i0, int i1, int* list, int* count) {
   const int lane = threadIdx.x & 31;
@@ -3003,7 +3015,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KP
   timeline(P, 1);
   const int inverted = ld_i(&P.st->inverted);
   if (inverted == 0) phase_lawson<true, true>(g, P, 0, stamp, lc, sc0);
-  else if (P.substeps > 0 || (sparse && P.V_it > kStarSparse) || !star_step<false>(g, P, stamp, q0, sc0, lc))
+  else if (P.substeps > 0 || P.V_it > kStarMost || (sparse && P.V_it > kStarSparse) || !star_step<false>(g, P, stamp, q0, sc0, lc))
     stamp = repair_step(g, P, stamp, q0);
   flush_counters(P, lc);
   // No closing grid barrier: each block leaves when its own work is done and
