@@ -2928,9 +2928,13 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
         break;
       }
       cs = stamp++;
-      if (gtid == 0) cnt[(slot + 1) % 3] = 0;
       int* next = lists[slot & 1];
       int* count = cnt + slot % 3;
+      // before anything joins (and of one mind with the blocks that already add to it):
+      // an append to a count that holds the bit is taken for a list that is full, an
+      // error of the step
+      if (ld_i(count) & kStarGivenUp) return false;
+      if (gtid == 0) cnt[(slot + 1) % 3] = 0;
       int inner;
       unsigned long long ranks;
       if (many) {
@@ -2952,7 +2956,6 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
       }
       g.sync();
       n = ld_i(count);
-      if (n >= kStarGivenUp || n < 0) return false;
       if (n == 0) ++slot;
     }
     touched = all_few ? ts : 0;
