@@ -175,7 +175,9 @@ int mcl_mesh_last_status(mcl_mesh* m, void* stream, mcl_step_stats* stats_host);
  * around every vertex, in the layout given; at most M-1 neighbours are stored
  * (the reference's truncation, include/kernels.cuh:68).  Order: clockwise
  * (the reference's PREV_OUTGOING walk), starting at the smallest neighbour id.
- * *truncated_host (may be NULL) receives the number of truncated vertices. */
+ * *truncated_host (may be NULL) receives the number of truncated vertices.
+ * This call, mcl_mesh_frnn, mcl_batch_frnn and the _list forms may overlap on one
+ * mesh, each on its own stream, from several threads. */
 int mcl_one_ring(mcl_mesh* m, int layout, int max_ring, int32_t* ring_dev, void* stream,
                  int64_t* truncated_host);
 

@@ -3373,7 +3373,8 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   // the mirror of the device state, behind it the counts that queries write and a step's
   // record: pages of the host's, pinned in place
   if (e == cudaSuccess) {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE), bytes = (sizeof(DevState) + 64 + sizeof(mcl_step_stats) + page - 1) / page * page;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), 
+                 bytes = (sizeof(DevState) + 8 * kCountSlots + sizeof(mcl_step_stats) + page - 1) / page * page;
     m->st_host = static_cast<DevState*>(std::aligned_alloc(page, bytes));
     e = m->st_host ? cudaHostRegister(m->st_host, bytes, cudaHostRegisterMapped) : cudaErrorMemoryAllocation;
   }
@@ -3381,8 +3382,8 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&m->counts_dev, m->counts_host, 0);
   static_assert(sizeof(DevState) % 8 == 0, "what follows the state in the mirror's pages");
   if (e == cudaSuccess) {
-    m->stats_host = reinterpret_cast<mcl_step_stats*>(m->counts_host + 8);
-    m->stats_map = reinterpret_cast<mcl_step_stats*>(m->counts_dev + 8);
+    m->stats_host = reinterpret_cast<mcl_step_stats*>(m->counts_host + kCountSlots);
+    m->stats_map = reinterpret_cast<mcl_step_stats*>(m->counts_dev + kCountSlots);
   }
   if (e != cudaSuccess) {
     (void)cudaGetLastError();

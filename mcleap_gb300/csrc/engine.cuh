@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <string>
+#include <thread>
 
 #include "predicates.cuh"
 #include "../../include/mcl_gb300.h"
@@ -379,8 +380,9 @@ struct mcl_mesh {
   mcl_step_stats* stats_dev;  // [2] published counters of the pipelined steps
   int stage_idx;
   unsigned long long* scratch;  // small device scratch for query counters (kScratchBytes)
-  unsigned long long* counts_host;  // behind st_host: counts of the last counted queries
+  unsigned long long* counts_host;  // behind st_host: counts of the counted queries in flight (kCountSlots)
   unsigned long long* counts_dev;   // the same, as the device sees them
+  unsigned count_slots;             // ... which of them are taken (CountSlot)
   mcl_step_stats* stats_host;       // behind those: the record a step writes when its caller waits for it
   mcl_step_stats* stats_map;        // ... as the device sees it
   mcl::DevState* st;
@@ -440,6 +442,35 @@ struct mcl_mesh {
 // Host-side helpers shared by the translation units of the library.
 namespace mcl {
 constexpr int kScratchBytes = 256;
+
+// A place for the counts of a query that is in flight, one of kCountSlots of its mesh:
+// queries of one mesh may overlap (several threads, each with its stream), and a kernel
+// that finds its counters clear and leaves them clear must not share them.  `taken` is
+// the mesh's word of bits; with all of them set the caller waits for one to return.
+constexpr int kCountSlots = 8;
+class CountSlot {
+ public:
+  explicit CountSlot(unsigned* taken) : taken_(taken) {
+    for (;;) {
+      unsigned t = __atomic_load_n(taken, __ATOMIC_RELAXED);
+      const unsigned free = ~t & ((1u << kCountSlots) - 1u);
+      if (!free) {
+        std::this_thread::yield();
+        continue;
+      }
+      at = __builtin_ctz(free);
+      if (__atomic_compare_exchange_n(taken, &t, t | 1u << at, false, __ATOMIC_ACQUIRE, __ATOMIC_RELAXED)) return;
+    }
+  }
+  ~CountSlot() { __atomic_fetch_and(taken_, ~(1u << at), __ATOMIC_RELEASE); }
+  CountSlot(const CountSlot&) = delete;
+  CountSlot& operator=(const CountSlot&) = delete;
+  int at;
+
+ private:
+  unsigned* taken_;
+};
+
 int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out);
 void free_mesh(mcl_mesh* m);
 int fail(int code, const std::string& msg);

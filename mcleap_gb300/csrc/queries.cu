@@ -64,8 +64,8 @@ constexpr int kMaxDeg = 4096;
 // kernel adds to cell[0], and its last block writes the sum to pinned host memory
 // and leaves the cell at zero for the next call, so that a query is one launch and
 // one wait (a memset before and a copy after it cost a small query as much as the
-// kernel).  cell[1] counts the blocks that have finished.  A call that asks for no
-// count passes no cell.
+// kernel).  cell[1] counts the blocks that have finished; the cell is the call's own
+// while it is in flight (CountSlot).  A call that asks for no count passes no cell.
 __device__ __forceinline__ void count_done(unsigned long long* cell, unsigned long long* host) {
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1055,18 +1055,28 @@ __global__ void k_debug_pred(int kind, const float* pts, const int* ids, int64_t
 
 namespace {
 
-// Counted queries: a cell pair per kind in the mesh's device scratch, a slot per
-// kind in its pinned host memory (count_done).
-enum { kCellRing = 8, kCellFrnn = 10, kHostRing = 0, kHostFrnn = 1 };
+// Counted queries: a cell pair per slot in the mesh's device scratch, a word per slot in
+// its pinned host memory (count_done).
+constexpr int kCells = 8;
+static_assert((kCells + 2 * kCountSlots) * 8 <= kScratchBytes, "the cells fit the scratch");
 
 MeshView mesh_view(const mcl_mesh* m) {
   return MeshView{m->ev, m->en, m->vhe, m->pos[m->cur], (int)m->V, (int)m->E};
 }
 
-int wait_count(unsigned long long* host, cudaStream_t s, int64_t* out) {
-  if (!out) return MCL_OK;
+// launch(cell, host): the query's kernel with the cell pair and the host word of its count.
+template <typename Launch>
+int counted(mcl_mesh* m, cudaStream_t s, int64_t* out, Launch launch) {
+  if (!out) {
+    launch(nullptr, nullptr);
+    QCK(cudaGetLastError());
+    return MCL_OK;
+  }
+  const CountSlot slot(&m->count_slots);
+  launch(m->scratch + kCells + 2 * slot.at, m->counts_dev + slot.at);
+  QCK(cudaGetLastError());
   QCK(cudaStreamSynchronize(s));
-  *out = (int64_t) * (volatile unsigned long long*)host;
+  *out = (int64_t) * (volatile unsigned long long*)(m->counts_host + slot.at);
   return MCL_OK;
 }
 
@@ -1079,13 +1089,10 @@ int launch_one_ring(mcl_mesh* m, const int* verts, int64_t n, int layout, int ma
   }
   const unsigned blocks = (unsigned)((n + kRingThreads - 1) / kRingThreads);
   const int delaunay = m->delaunay && m->valid_cur ? 1 : 0;
-  unsigned long long* host = truncated ? m->counts_host + kHostRing : nullptr;
   auto kernel = layout == MCL_LAYOUT_COLUMN ? k_one_ring<false> : k_one_ring<true>;
-  kernel<<<blocks, kRingThreads, 0, s>>>(mesh_view(m), verts, (int)n, max_ring, out, m->vfix, delaunay,
-                                         host ? m->scratch + kCellRing : nullptr,
-                                         host ? m->counts_dev + kHostRing : nullptr);
-  QCK(cudaGetLastError());
-  return wait_count(host, s, truncated);
+  return counted(m, s, truncated, [&](unsigned long long* cell, unsigned long long* host) {
+    kernel<<<blocks, kRingThreads, 0, s>>>(mesh_view(m), verts, (int)n, max_ring, out, m->vfix, delaunay, cell, host);
+  });
 }
 
 int launch_mesh_frnn(mcl_mesh* m, const int* verts, int64_t n, float r2, const float* rcomp, int layout, int max_frnn,
@@ -1095,13 +1102,11 @@ int launch_mesh_frnn(mcl_mesh* m, const int* verts, int64_t n, float r2, const f
     if (overflow) *overflow = 0;
     return MCL_OK;
   }
-  unsigned long long* host = overflow ? m->counts_host + kHostFrnn : nullptr;
   constexpr int kPer = 32 / kFrnnLanes * kFrnnWarps;
-  k_mesh_frnn<<<(unsigned)((n + kPer - 1) / kPer), 32 * kFrnnWarps, 0, s>>>(
-      mesh_view(m), verts, (int)n, r2, layout, max_frnn, out, host ? m->scratch + kCellFrnn : nullptr,
-      host ? m->counts_dev + kHostFrnn : nullptr, rcomp, rcomp ? m->vcomp : nullptr);
-  QCK(cudaGetLastError());
-  return wait_count(host, s, overflow);
+  return counted(m, s, overflow, [&](unsigned long long* cell, unsigned long long* host) {
+    k_mesh_frnn<<<(unsigned)((n + kPer - 1) / kPer), 32 * kFrnnWarps, 0, s>>>(
+        mesh_view(m), verts, (int)n, r2, layout, max_frnn, out, cell, host, rcomp, rcomp ? m->vcomp : nullptr);
+  });
 }
 
 }  // namespace
