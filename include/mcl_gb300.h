@@ -491,7 +491,9 @@ int mcl_periodic_debug_timeline(const mcl_periodic* m, int64_t* out32, int64_t* 
  * MCL_LAYOUT_COLUMN (ring[(k+1) n + i]) or MCL_LAYOUT_ROW (ring[i max_ring + k]).
  * offs_dev (may be NULL; same layout, one byte per slot) receives each
  * neighbour's copy offset relative to the vertex (an offset byte as in eo).
- * truncated (may be NULL): vertices with more than max_ring - 1 neighbours. */
+ * truncated (may be NULL): vertices with more than max_ring - 1 neighbours.
+ * Once one such call has returned since the last step, others may overlap, each
+ * on its own stream, from several threads. */
 int mcl_periodic_one_ring(mcl_periodic* m, int max_ring, int layout, int32_t* ring_dev, uint8_t* offs_dev,
                           void* stream, int64_t* truncated);
 

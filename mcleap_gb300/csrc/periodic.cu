@@ -68,8 +68,9 @@ struct mcl_periodic {
   unsigned long long* claim;
   int* vhe;          // one outgoing half-edge per vertex (queries), kept by the steps' flips
   bool vhe_ok;       // ... since a query last worked them out
-  PCount* cnt;       // a query's counters; then the ring's, clear between calls, and its ticket
-  PCount* cnt_host;  // pinned
+  PCount* cnt;       // a query's counters; then the ring queries' by slot, clear between calls, and tickets
+  PCount* cnt_host;  // pinned: a query's; then the ring queries' by slot
+  unsigned count_slots;  // slots taken by ring queries in flight (CountSlot)
   unsigned stamp;    // last round stamp used
   // the step's cooperative launch (allocated on the first step)
   PCount* slots;     // three rotating phase counters, clear between launches
@@ -737,6 +738,9 @@ __global__ void k_pclosest(PView V, bool column, int max_ring, const int* ring, 
   if (i < V.n) mcl::p_body_closest(V, i, column, max_ring, ring, offs, out);
 }
 
+// The query's counters, the ring queries' and their tickets.
+constexpr size_t kCountBytes = (1 + mcl::kCountSlots) * sizeof(PCount) + 4 * mcl::kCountSlots;
+
 unsigned blocks(int64_t k) { return (unsigned)((k + kThreads - 1) / kThreads); }
 
 PView view(mcl_periodic* m) {
@@ -968,8 +972,8 @@ int alloc_upload(const mcl_float2* pos, int64_t n, float L, const int32_t* ev, c
   A((void**)&m->cand, 4 * (size_t)E);
   A((void**)&m->claim, 16 * (size_t)E);
   A((void**)&m->vhe, 4 * (size_t)n);
-  A((void**)&m->cnt, 2 * sizeof(PCount) + 8);
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&m->cnt_host, sizeof(PCount));
+  A((void**)&m->cnt, kCountBytes);
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&m->cnt_host, (1 + mcl::kCountSlots) * sizeof(PCount));
   if (e == cudaSuccess) e = cudaMemcpy(m->pos, pos, 8 * (size_t)n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(m->ev, ev, 16 * (size_t)E, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(m->en, en, 16 * (size_t)E, cudaMemcpyHostToDevice);
@@ -982,7 +986,7 @@ int alloc_upload(const mcl_float2* pos, int64_t n, float L, const int32_t* ev, c
   if (e == cudaSuccess) e = cudaMemset(m->cand, 0, 4 * (size_t)E);
   if (e == cudaSuccess) e = cudaMemset(m->claim, 0, 16 * (size_t)E);
   if (e == cudaSuccess) e = cudaMemset(m->qstamp, 0, 4 * (size_t)E);
-  if (e == cudaSuccess) e = cudaMemset(m->cnt, 0, 2 * sizeof(PCount) + 8);
+  if (e == cudaSuccess) e = cudaMemset(m->cnt, 0, kCountBytes);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     free_periodic(m);
@@ -1249,21 +1253,23 @@ int mcl_periodic_one_ring(mcl_periodic* m, int max_ring, int layout, int32_t* ri
   if (!m || !ring_dev || max_ring < 1 || (layout != MCL_LAYOUT_COLUMN && layout != MCL_LAYOUT_ROW))
     return mcl::fail(MCL_ERR_INVALID_ARGUMENT, "mcl_periodic_one_ring: bad arguments");
   cudaStream_t s = (cudaStream_t)stream;
+  const mcl::CountSlot slot(&m->count_slots);
+  PCount* host = m->cnt_host + 1 + slot.at;
   PView V = view(m);
-  V.cnt = m->cnt + 1;
+  V.cnt = m->cnt + 1 + slot.at;
   if (!m->vhe_ok) {
     PCK(cudaMemsetAsync(m->vhe, 0xFF, 4 * (size_t)m->n, s));  // vhe = -1: the largest candidate wins
     k_pvhe<<<blocks(2 * m->E), kThreads, 0, s>>>(V, m->vhe);
   }
   k_pring<<<blocks(m->n), kThreads, 0, s>>>(V, layout == MCL_LAYOUT_COLUMN, max_ring, ring_dev, offs_dev,
-                                            reinterpret_cast<unsigned*>(m->cnt + 2), m->cnt_host);
+                                            reinterpret_cast<unsigned*>(m->cnt + 1 + mcl::kCountSlots) + slot.at, host);
   PCK(cudaGetLastError());
   PCK(cudaStreamSynchronize(s));
-  m->vhe_ok = m->cnt_host->error == 0;
-  if (m->cnt_host->error)
-    return mcl::fail((int)m->cnt_host->error,
-                     "mcl_periodic_one_ring: malformed mesh (site " + std::to_string(m->cnt_host->error_site) + ")");
-  if (truncated) *truncated = (int64_t)m->cnt_host->truncated;
+  m->vhe_ok = host->error == 0;
+  if (host->error)
+    return mcl::fail((int)host->error,
+                     "mcl_periodic_one_ring: malformed mesh (site " + std::to_string(host->error_site) + ")");
+  if (truncated) *truncated = (int64_t)host->truncated;
   return MCL_OK;
 }
 

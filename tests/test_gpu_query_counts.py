@@ -1,11 +1,11 @@
-"""Counted queries of one mesh from several threads, each on its own stream: every
+"""Counted queries of one mesh or torus from several threads, each on its own stream: every
 call's count is that of the same call alone, during the overlap and after it."""
 import threading
 
 import numpy as np
 import pytest
 
-from helpers import uniform_points
+from helpers import torus_points, uniform_points
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +70,26 @@ def test_mesh_queries_overlap(M, threads):
         assert got == [alone[i]] * 200, i
     assert [j() for j in jobs] == alone
     b.close()
+
+
+@pytest.mark.parametrize("threads", [2, 5])
+def test_torus_rings_overlap(M, threads):
+    import torch
+
+    t = M.PeriodicTriangulation(torus_points(3000, 9))
+    first = torch.empty(t.n * 16, dtype=torch.int32, device="cuda")
+    t.oneRing(16, first)  # works out the half-edges that later calls start from
+
+    def job(i):
+        s = torch.cuda.Stream()
+        out = torch.empty(t.n * 16, dtype=torch.int32, device="cuda")
+        return lambda: t.oneRing(6 + i, out, stream=s)
+
+    jobs = [job(i) for i in range(threads)]
+    torch.cuda.synchronize()
+    alone = [j() for j in jobs]
+    assert alone[0] > 0
+    for i, got in enumerate(together(jobs, 200)):
+        assert got == [alone[i]] * 200, i
+    assert [j() for j in jobs] == alone
+    t.close()
