@@ -354,6 +354,7 @@ int mcl_batch_create(mcl_mesh* const* meshes, int64_t count, mcl_mesh** out) {
       cudaMalloc((void**)&b->cebase, 4 * count) != cudaSuccess)
     return bail(fail(MCL_ERR_OUT_OF_MEMORY, "mcl_batch_create: component tables"));
   b->ncomp = count;
+  b->square = true;
   b->comp_host = new int64_t[4 * count];
   std::vector<int> base((size_t)count + 1), ebase((size_t)count);
   b->T = 0;
@@ -372,6 +373,7 @@ int mcl_batch_create(mcl_mesh* const* meshes, int64_t count, mcl_mesh** out) {
                                        b->vcomp, b->vroot);
     if (cudaGetLastError() != cudaSuccess) return bail(fail(MCL_ERR_CUDA, "mcl_batch_create: append"));
     b->T += m->T;
+    b->square = b->square && m->square;
     vb += m->V;
     eb += m->E;
   }
@@ -447,6 +449,7 @@ int mcl_mesh_clone(const mcl_mesh* src, mcl_mesh** out) {
     return cuda_fail(e, "mcl_mesh_clone");
   }
   m->T = src->T;
+  m->square = src->square;
   m->ncomp = src->ncomp;
   if (src->comp_host) {
     m->comp_host = new int64_t[4 * src->ncomp];

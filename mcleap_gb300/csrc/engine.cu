@@ -3018,7 +3018,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KP
   timeline(P, 1);
   const int inverted = ld_i(&P.st->inverted);
   if (inverted == 0) phase_lawson<true, true>(g, P, 0, stamp, lc, sc0);
-  else if (P.substeps > 0 || P.V_it > kStarMost || (sparse && P.V_it > kStarSparse) || !star_step<false>(g, P, stamp, q0, sc0, lc))
+  else if (P.substeps > 0 || !P.square || P.V_it > kStarMost || (sparse && P.V_it > kStarSparse) || !star_step<false>(g, P, stamp, q0, sc0, lc))
     stamp = repair_step(g, P, stamp, q0);
   flush_counters(P, lc);
   // No closing grid barrier: each block leaves when its own work is done and
@@ -3461,6 +3461,20 @@ static bool aos_to_soa(const mcl_aos_view* a, std::vector<int4>& ev, std::vector
   return true;
 }
 
+// mcl_mesh::square of a mesh that aos_to_soa has accepted.
+static bool has_square(const mcl_aos_view* a) {
+  int64_t border = 0;
+  for (int64_t h = 0; h < a->HE; ++h) {
+    if (a->he[4 * h + 2] >= 0) continue;
+    const int from = a->he[4 * h + 1], to = a->he[4 * (h ^ 1) + 1];
+    if (from > 3 || to != ((from + 3) & 3)) return false;
+    ++border;
+  }
+  const mcl_float2* p = a->pos;
+  return border == 4 && p[0].x < p[1].x && p[1].y < p[2].y && p[0].y == p[1].y && p[1].x == p[2].x &&
+         p[2].y == p[3].y && p[3].x == p[0].x;
+}
+
 static int upload_soa(mcl_mesh* m, const mcl_float2* pos, const std::vector<int4>& ev, const std::vector<int4>& en,
                       const std::vector<int>& vhe) {
   std::vector<unsigned char> fix(m->V, 0);
@@ -3704,6 +3718,7 @@ static int run_step(mcl_mesh* m, int move_mode, const float2* d, cudaStream_t s,
     P.pos_old = m->valid_cur ? m->pos[m->cur] : m->pos[m->cur ^ 1];
   }
   P.sparse_ok = m->delaunay ? 1 : 0;
+  P.square = m->square ? 1 : 0;
   int rc = launch_engine(m, P, s);
   if (rc != MCL_OK) return rc;
   m->valid_cur = true;
@@ -3876,6 +3891,7 @@ int mcl_mesh_create_from_aos(const mcl_aos_view* a, mcl_mesh** out) {
   rc = upload_soa(m, a->pos, ev, en, vhe);
   if (rc != MCL_OK) { free_mesh(m); return rc; }
   m->delaunay = false;  // a caller's mesh: the first step classifies every edge
+  m->square = has_square(a);
   *out = m;
   return MCL_OK;
 }
@@ -3888,6 +3904,7 @@ int mcl_mesh_upload_aos(mcl_mesh* m, const mcl_aos_view* a) {
   std::string why;
   if (!aos_to_soa(a, ev, en, vhe, why)) return fail(MCL_ERR_INVALID_ARGUMENT, "malformed mesh: " + why);
   m->delaunay = false;
+  m->square = has_square(a);
   return upload_soa(m, a->pos, ev, en, vhe);
 }
 
@@ -4056,6 +4073,7 @@ int mcl_mesh_build(mcl_float2* pts, int64_t n, mcl_mesh** out) {
   mcl_mesh* m = nullptr;
   int rc = alloc_mesh(V, E, &m);
   if (rc != MCL_OK) return rc;
+  m->square = true;
   KParams P = make_params(m, ENGINE_BUILD);
   P.pos = m->pos[0];
   P.pos_old = m->pos[0];

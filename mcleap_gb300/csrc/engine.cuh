@@ -167,6 +167,7 @@ struct KParams {
   int tail_items;          // flip rounds with at most this many queued edges run in one block
   int rm_tile;             // lanes of a warp that take removal-list entries (0: as few as fit one pass)
   int substeps;            // repair sub-steps before removal
+  int square;              // the first four vertices of every mesh are its square's corners (mcl_mesh::square)
   int sparse_ok;           // the mesh is Delaunay at pos_old: a step may classify only its movers' stars
   int append_marks;        // repair: append marked edges to work-list 0 (few removals), else rebuild from the marks
   mcl_step_stats* stats_out;  // device-visible host record the launch fills at its end (or NULL)
@@ -398,6 +399,11 @@ struct mcl_mesh {
   bool tail_auto;          // ... not set by the caller: at most one edge per thread
   int rm_tile;             // removal tile (mcl_mesh_set_removal_tile; 0 = automatic)
   int substeps;            // repair sub-steps before removal (mcl_mesh_set_substeps)
+  // the first four vertices (of every mesh) are the corners of an upright rectangle,
+  // counter-clockwise from the lower left, and its sides are the whole border: what
+  // untangling by stars and the corners' rings start from.  An imported mesh may be
+  // another triangulation; it is stepped and queried without them.
+  bool square;
   bool delaunay;           // the last launch left the mesh Delaunay (set when a step or build is launched)
   // batches: a mesh made of independent components (mcl_batch_create)
   int64_t ncomp;           // 1 for a plain mesh

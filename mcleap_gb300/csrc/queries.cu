@@ -136,8 +136,8 @@ __device__ __noinline__ void ring_walk(const MeshView M, int h0, int cap, size_t
   if (truncated && deg > cap) atomicAdd(truncated, 1ull);
 }
 
-// Rows for the vertices verts[0 .. n) (NULL: all of them).  delaunay: the mesh is a
-// Delaunay triangulation; vfix marks the corners.
+// Rows for the vertices verts[0 .. n) (NULL: all of them).  delaunay: the mesh is the
+// Delaunay triangulation of its square; vfix marks the corners.
 template <bool kRow>
 __global__ void __launch_bounds__(kRingThreads) k_one_ring(MeshView M, const int* __restrict__ verts, int n,
                                                            int max_ring, int* ring,
@@ -1088,7 +1088,7 @@ int launch_one_ring(mcl_mesh* m, const int* verts, int64_t n, int layout, int ma
     return MCL_OK;
   }
   const unsigned blocks = (unsigned)((n + kRingThreads - 1) / kRingThreads);
-  const int delaunay = m->delaunay && m->valid_cur ? 1 : 0;
+  const int delaunay = m->delaunay && m->valid_cur && m->square ? 1 : 0;
   auto kernel = layout == MCL_LAYOUT_COLUMN ? k_one_ring<false> : k_one_ring<true>;
   return counted(m, s, truncated, [&](unsigned long long* cell, unsigned long long* host) {
     kernel<<<blocks, kRingThreads, 0, s>>>(mesh_view(m), verts, (int)n, max_ring, out, m->vfix, delaunay, cell, host);
