@@ -326,8 +326,9 @@ int mcl_mesh_clone(const mcl_mesh* src, mcl_mesh** out);
 
 /* Launch shape of the kinetic step: blocks_per_sm in [1, max] (0 = max), and
  * the work-list size at or below which one block finishes the flip rounds
- * (0 = 2048, and no more edges than the block has threads).  Results do not
- * depend on either. */
+ * (0 = 256, an edge for each thread of the block).  Results do not depend on
+ * either.  mcl_mesh_get_tuning gives the values in use; setting them again
+ * changes nothing. */
 int mcl_mesh_set_tuning(mcl_mesh* m, int blocks_per_sm, int tail_items);
 /* Work-list tile of the repair's removal rounds: how many lanes of each warp
  * take entries of the vertex list (1..32; 0 = automatic, as few as let one

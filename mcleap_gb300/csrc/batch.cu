@@ -456,7 +456,6 @@ int mcl_mesh_clone(const mcl_mesh* src, mcl_mesh** out) {
     std::memcpy(m->comp_host, src->comp_host, sizeof(int64_t) * 4 * src->ncomp);
   }
   m->tail_items = src->tail_items;
-  m->tail_auto = src->tail_auto;
   m->rm_tile = src->rm_tile;
   m->coop_blocks = src->coop_blocks;
   if (src->substeps > 0 && (rc = mcl_mesh_set_substeps(m, src->substeps)) != MCL_OK) {
@@ -525,8 +524,7 @@ int mcl_mesh_set_tuning(mcl_mesh* m, int blocks_per_sm, int tail_items) {
   if (bps > m->max_blocks_per_sm)
     return fail(MCL_ERR_INVALID_ARGUMENT, "blocks per SM above the kernel's co-resident limit");
   m->coop_blocks = m->nsm * bps;
-  m->tail_items = tail_items == 0 ? 2048 : tail_items;
-  m->tail_auto = tail_items == 0;
+  m->tail_items = tail_items == 0 ? kTailItems : tail_items;
   return MCL_OK;
 }
 

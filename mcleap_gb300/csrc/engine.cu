@@ -733,12 +733,12 @@ __device__ __forceinline__ int lawson_round(const KParams& P, const int* in, int
 }
 
 // Rounds with at most this many queued edges run inside one block (block
-// barriers instead of grid barriers); the rest of the grid waits.  Left to itself a
-// mesh takes no more than the block has threads: a second pass over the list waits for
-// the loads of the first (20,000 points advected: 1600 edges in one block 18 us, over
-// the grid with two grid barriers 8; the step's launch 54 -> 43 us; limits of 32 to 384
-// the same within 2 us, 512 and above 54).
-constexpr int kTailItems = 2048;
+// barriers instead of grid barriers); the rest of the grid waits.  No more than the
+// block has threads: a second pass over the list waits for the loads of the first
+// (20,000 points advected: 1600 edges in one block 18 us, over the grid with two grid
+// barriers 8; the step's launch 54 -> 43 us; limits of 32 to 384 the same within 2 us,
+// 512 and above 54).
+static_assert(kTailItems == kThreads, "an edge per thread");
 // Default repair sub-steps per kinetic step (phase_substeps).  Off: on the
 // uniform random-walk benchmarks (1M points, sigma = 0.1 x spacing; 512 meshes,
 // 8.5M points) 4 and 8 sub-steps leave 25% and 4% of the sent-back vertices
@@ -3411,7 +3411,6 @@ int alloc_mesh(int64_t V, int64_t E, mcl_mesh** out) {
   m->nsm = nsm;
   m->max_blocks_per_sm = per_sm;
   m->tail_items = kTailItems;
-  m->tail_auto = true;
   m->substeps = kSubsteps;
   m->ncomp = 1;
   m->coop_blocks = nsm * per_sm;
@@ -3608,7 +3607,7 @@ static KParams make_params(mcl_mesh* m, int mode) {
   P.mode = mode;
   P.max_rounds = 1 << 16;
   P.walk_cap = 1 << 18;
-  P.tail_items = m->tail_auto ? std::min(kTailItems, kThreads) : m->tail_items;
+  P.tail_items = m->tail_items;
   P.rm_tile = m->rm_tile;
   P.substeps = m->vl2 ? m->substeps : 0;  // no scratch, no sub-steps
   P.vroot = m->vroot;

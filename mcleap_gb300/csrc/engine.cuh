@@ -395,8 +395,7 @@ struct mcl_mesh {
   // tuning (mcl_mesh_set_tuning)
   int nsm;                 // SMs of the device
   int max_blocks_per_sm;   // k_step occupancy limit
-  int tail_items;          // single-block flip-round threshold
-  bool tail_auto;          // ... not set by the caller: at most one edge per thread
+  int tail_items;          // single-block flip-round threshold (kTailItems unless the caller set one)
   int rm_tile;             // removal tile (mcl_mesh_set_removal_tile; 0 = automatic)
   int substeps;            // repair sub-steps before removal (mcl_mesh_set_substeps)
   // the first four vertices (of every mesh) are the corners of an upright rectangle,
@@ -448,6 +447,7 @@ struct mcl_mesh {
 // Host-side helpers shared by the translation units of the library.
 namespace mcl {
 constexpr int kScratchBytes = 256;
+constexpr int kTailItems = 256;  // a flip round's edges up to which one block takes it, by default
 
 // A place for the counts of a query that is in flight, one of kCountSlots of its mesh:
 // queries of one mesh may overlap (several threads, each with its stream), and a kernel
