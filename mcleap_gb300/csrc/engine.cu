@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstddef>
 #include <cstdio>
 #include <cstdlib>
@@ -193,6 +194,7 @@ __device__ void flush_counters(const KParams& P, LocalCounters& lc) {
   // per warp on a single address cost microseconds at the end of every step),
   // atomics for the rare ones
   __shared__ unsigned long long part[kThreads / 32];
+  __syncthreads();  // one flush may follow another: the sums of the last have been read
   unsigned long long inc = lc.incircle;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) inc += __shfl_down_sync(kFull, inc, o);
@@ -920,9 +922,13 @@ __device__ void mark_face(const KParams& P, int a, int b, int c, int& fresh, uns
   }
 }
 
-__device__ bool phase_fixpoint(cg::grid_group& g, const KParams& P, LocalCounters& lc, unsigned fs) {
+// Returns MCL_OK, an error, or kSentBackMany once more than `most` vertices have been
+// marked (listed again ones counted too).
+constexpr int kSentBackMany = -1;
+__device__ int phase_fixpoint(cg::grid_group& g, const KParams& P, LocalCounters& lc, unsigned fs, long long most) {
   const int stride = gridDim.x * blockDim.x;
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  long long all = 0;  // of the passes so far, the same in every thread (fix_all moves on)
   for (int pass = 0; pass < 256; ++pass) {
     // counters are triple-buffered: slot (pass+1)%3 was last read two barriers ago
     const int slot = pass % 3;
@@ -997,16 +1003,11 @@ __device__ bool phase_fixpoint(cg::grid_group& g, const KParams& P, LocalCounter
     if (pass < 16) timeline_remove(P, 48 + pass);
     const int nfresh = ld_i(&P.st->fix_new[slot]);
     const int nbad = ld_i(&P.st->fix_bad[slot]);
-    if (nfresh == 0) {
-      if (nbad) {
-        if (gtid == 0) set_error(P, MCL_ERR_DEGENERATE_INPUT);
-        return false;
-      }
-      return true;
-    }
+    if (nfresh == 0) return nbad ? MCL_ERR_DEGENERATE_INPUT : MCL_OK;
+    all += nfresh;
+    if (all > most) return kSentBackMany;
   }
-  if (gtid == 0) set_error(P, MCL_ERR_NO_CONVERGENCE);
-  return false;
+  return MCL_ERR_NO_CONVERGENCE;
 }
 
 // ---------------------------------------------------------------------------
@@ -2108,17 +2109,40 @@ __device__ void phase_substeps(cg::grid_group& g, const KParams& P, unsigned& st
   g.sync();
 }
 
-// Repair of a step whose classification found inverted faces: revert, remove,
-// Lawson, reinsert.  Out of line, so k_step's hot loops keep their registers;
-// keeps its own counters and returns the next free stamp.
-__device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, unsigned stamp, unsigned q0) {
+// The removal path's first part, for a step whose classification found inverted faces:
+// the vertices to send back, marked with fs.  The mesh is as it was when it returns.
+__device__ __noinline__ int send_back(cg::grid_group g, const KParams P, unsigned fs, long long most) {
+  LocalCounters lc = {0, 0, 0, 0, 0, 0, 0};
+  KParams Q = P;
+  Q.move_mode = MOVE_NONE;  // positions were moved by the classification
+  const int rc = phase_fixpoint(g, Q, lc, fs, most);
+  flush_counters(P, lc);
+  return rc;
+}
+
+// The rest of it: remove the vertices sent back (fs), reinsert them at the new positions,
+// Lawson.  Out of line, so k_step's hot loops keep their registers; keeps its own
+// counters and returns the next free stamp.  fs = 0: nothing has been sent back yet, or a
+// send-back was given up.
+__device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, unsigned stamp, unsigned q0,
+                                             unsigned fs) {
+  if (fs == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      for (int i = 0; i < 3; ++i) P.st->fix_new[i] = P.st->fix_bad[i] = P.st->fix_list[i] = 0;
+      P.st->fix_all = 0;
+    }
+    g.sync();
+    fs = stamp++;
+    const int rc = send_back(g, P, fs, LLONG_MAX);
+    if (rc != MCL_OK) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) set_error(P, rc);
+      return stamp;
+    }
+  }
   LocalCounters lc = {0, 0, 0, 0, 0, 0, 0};
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
   KParams Q = P;
-  Q.move_mode = MOVE_NONE;  // positions were moved by the classification
-  const int inverted = ld_i(&P.st->inverted);
-  if (gtid == 0) P.st->c[C_INVERTED] += (unsigned long long)inverted;
-  const unsigned fs = stamp++;  // revert marks of this launch
+  Q.move_mode = MOVE_NONE;
   // Edges to pass through Lawson at the end carry the mark mk: the
   // classification's non-Delaunay edges (queued with q0), then every edge a
   // removal or a split touches.  Any other edge is Delaunay: its quad keeps
@@ -2126,150 +2150,147 @@ __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, 
   // and each edge whose quad held one is a spoke, gone, or a side of its
   // hole, marked).
   unsigned mk = q0;
-  // (1) revert until valid
-  bool ok = phase_fixpoint(g, Q, lc, fs);
+  bool ok = true;
   g.sync();
   timeline(P, 43);
-  if (ok) {
-    // removal list: reverted vertices that actually moved.  Few: from the
-    // list of every vertex sent back (on `hard`); many: by a pass over the
-    // vertices, whose id order keeps neighbouring removals in one warp
-    // (the mark order scatters them).
-    const int stride = gridDim.x * blockDim.x;
-    const int nall = ld_i(&P.st->fix_all);
-    const bool few = (long long)nall * 64 < (long long)P.V_it;
+  // removal list: reverted vertices that actually moved.  Few: from the
+  // list of every vertex sent back (on `hard`); many: by a pass over the
+  // vertices, whose id order keeps neighbouring removals in one warp
+  // (the mark order scatters them).
+  const int stride = gridDim.x * blockDim.x;
+  const int nall = ld_i(&P.st->fix_all);
+  const bool few = (long long)nall * 64 < (long long)P.V_it;
+  if (gtid == 0) { P.st->vl_count[0] = 0; P.st->vl_count[1] = 0; }
+  g.sync();
+  const int nsb = few ? nall : P.V_it;
+  WarpBuf wrev{warp_buf(0), 0};
+  for (int base = (few ? spread_tid() - (int)(threadIdx.x & 31) : blockIdx.x * blockDim.x); base < nsb;
+       base += stride) {
+    const int vi = base + (few ? (int)(threadIdx.x & 31) : (int)threadIdx.x);
+    const int v = vi < nsb ? (few ? ld_i(P.hard + vi) : vert_at(P, vi)) : 0;
+    int mine[1];
+    int k = 0;
+    if (vi < nsb && marked(Q, v, fs) && !P.vfix[v]) {
+      const float2 pn = ldpos(Q, v), po = P.pos_old[v];
+      if (__float_as_uint(pn.x) != __float_as_uint(po.x) || __float_as_uint(pn.y) != __float_as_uint(po.y)) {
+        __stcg(P.target + v, pn);
+        __stcg(P.pos + v, po);
+        __stcg(P.vlocf + v, 0);  // sub-step level
+        mine[k++] = v;
+      }
+    }
+    wb_push(wrev, mine, k, P.vl0, &P.st->vl_count[0], P.V, P.st);
+  }
+  wb_flush(wrev, P.vl0, &P.st->vl_count[0], P.V, P.st);
+  g.sync();
+  const int nrev = ld_i(&P.st->vl_count[0]);
+  if (gtid == 0) P.st->c[C_REVERTED] += (unsigned long long)nrev;
+  if (nrev > 0 && P.substeps > 0) {
+    // (1b) Delaunay over every edge with the sent-back vertices at their old
+    // positions, then sub-steps toward their targets; the mesh is then
+    // Delaunay, so only what removal and reinsertion touch is marked
+    if (gtid == 0) { P.st->wl_count[0] = 0; P.st->wl_count[1] = 0; P.st->inverted = 0; P.st->hard_count = 0; }
+    g.sync();
+    const unsigned qa = stamp++;
+    const unsigned sc0 = stamp++;
+    phase_classify<false>(g, Q, qa, sc0, lc);
+    g.sync();
+    phase_classify_hard<false>(g, Q, qa, sc0, lc);
+    phase_lawson<false>(g, Q, 0, stamp, lc, sc0);
+    g.sync();
+    timeline_insert(P, 15, 0);
+    phase_substeps(g, Q, stamp, lc);
+    timeline_insert(P, 15, 1);
+    mk = stamp++;
+    // the mesh is Delaunay again: the final Lawson list starts empty
+    if (gtid == 0) { P.st->wl_count[0] = 0; P.st->wl_count[1] = 0; }
+    g.sync();
+  }
+  const int nrem = ld_i(&P.st->vl_count[0]);
+  // few removals: their marks are appended to a list (no pass over every
+  // edge afterwards); many: the list is rebuilt from the marks
+  Q.append_marks = (long long)nrem * 64 < (long long)P.E_it ? 1 : 0;
+  if (!Q.append_marks && gtid == 0) P.st->mark_ovf = 1;
+  if (nrem > 0) {
+    // (2) remove what is left, marking each hole's sides and diagonals
+    ok = phase_remove(g, Q, stamp, lc, mk);
+    g.sync();
+    timeline(P, 44);
+    // (3) reinsert at the new positions: splits only, their edges marked
     if (gtid == 0) { P.st->vl_count[0] = 0; P.st->vl_count[1] = 0; }
     g.sync();
-    const int nsb = few ? nall : P.V_it;
-    WarpBuf wrev{warp_buf(0), 0};
-    for (int base = (few ? spread_tid() - (int)(threadIdx.x & 31) : blockIdx.x * blockDim.x); base < nsb;
+    // the removed vertices: from the list of every vertex sent back when
+    // few (and the sub-steps' classification did not reuse its buffer),
+    // else by a pass over the vertices
+    const bool from_list = few && !(nrev > 0 && P.substeps > 0);
+    const int nscan = from_list ? nall : P.V_it;
+    WarpBuf wins{warp_buf(0), 0};
+    for (int base = (from_list ? spread_tid() - (int)(threadIdx.x & 31) : blockIdx.x * blockDim.x); base < nscan;
          base += stride) {
-      const int vi = base + (few ? (int)(threadIdx.x & 31) : (int)threadIdx.x);
-      const int v = vi < nsb ? (few ? ld_i(P.hard + vi) : vert_at(P, vi)) : 0;
+      const int vi = base + (from_list ? (int)(threadIdx.x & 31) : (int)threadIdx.x);
+      const int v = vi < nscan ? (from_list ? ld_i(P.hard + vi) : vert_at(P, vi)) : 0;
       int mine[1];
       int k = 0;
-      if (vi < nsb && marked(Q, v, fs) && !P.vfix[v]) {
-        const float2 pn = ldpos(Q, v), po = P.pos_old[v];
-        if (__float_as_uint(pn.x) != __float_as_uint(po.x) || __float_as_uint(pn.y) != __float_as_uint(po.y)) {
-          __stcg(P.target + v, pn);
-          __stcg(P.pos + v, po);
-          __stcg(P.vlocf + v, 0);  // sub-step level
-          mine[k++] = v;
-        }
+      if (vi < nscan && ld_i(P.vhe + v) < 0 && marked(Q, v, fs)) {
+        __stcg(P.pos + v, __ldcg(P.target + v));
+        mine[k++] = v;
       }
-      wb_push(wrev, mine, k, P.vl0, &P.st->vl_count[0], P.V, P.st);
+      wb_push(wins, mine, k, P.vl0, &P.st->vl_count[0], P.V, P.st);
     }
-    wb_flush(wrev, P.vl0, &P.st->vl_count[0], P.V, P.st);
+    wb_flush(wins, P.vl0, &P.st->vl_count[0], P.V, P.st);
     g.sync();
-    const int nrev = ld_i(&P.st->vl_count[0]);
-    if (gtid == 0) P.st->c[C_REVERTED] += (unsigned long long)nrev;
-    if (nrev > 0 && P.substeps > 0) {
-      // (1b) Delaunay over every edge with the sent-back vertices at their old
-      // positions, then sub-steps toward their targets; the mesh is then
-      // Delaunay, so only what removal and reinsertion touch is marked
-      if (gtid == 0) { P.st->wl_count[0] = 0; P.st->wl_count[1] = 0; P.st->inverted = 0; P.st->hard_count = 0; }
-      g.sync();
-      const unsigned qa = stamp++;
-      const unsigned sc0 = stamp++;
-      phase_classify<false>(g, Q, qa, sc0, lc);
-      g.sync();
-      phase_classify_hard<false>(g, Q, qa, sc0, lc);
-      phase_lawson<false>(g, Q, 0, stamp, lc, sc0);
-      g.sync();
-      timeline_insert(P, 15, 0);
-      phase_substeps(g, Q, stamp, lc);
-      timeline_insert(P, 15, 1);
-      mk = stamp++;
-      // the mesh is Delaunay again: the final Lawson list starts empty
+    if (ok) ok = phase_insert(g, Q, stamp, lc, mk);
+    g.sync();
+  } else {
+    timeline(P, 44);
+  }
+  timeline(P, 45);
+  // (4) one Lawson pass from every marked edge: work-list 0 holds the
+  // classification's non-Delaunay edges and the appended marks, repeats
+  // included; deduplicated into work-list 1 when short, else rebuilt from
+  // the marks over every edge
+  if (ok) {
+    const int nw = ld_i(&P.st->wl_count[0]);
+    const bool rebuild = ld_i(&P.st->mark_ovf) || (long long)nw * 4 >= (long long)P.E_it;
+    g.sync();  // every thread has read the count and the flag
+    if (rebuild) {
       if (gtid == 0) { P.st->wl_count[0] = 0; P.st->wl_count[1] = 0; }
       g.sync();
-    }
-    const int nrem = ld_i(&P.st->vl_count[0]);
-    // few removals: their marks are appended to a list (no pass over every
-    // edge afterwards); many: the list is rebuilt from the marks
-    Q.append_marks = (long long)nrem * 64 < (long long)P.E_it ? 1 : 0;
-    if (!Q.append_marks && gtid == 0) P.st->mark_ovf = 1;
-    if (nrem > 0) {
-      // (2) remove what is left, marking each hole's sides and diagonals
-      ok = phase_remove(g, Q, stamp, lc, mk);
-      g.sync();
-      timeline(P, 44);
-      // (3) reinsert at the new positions: splits only, their edges marked
-      if (gtid == 0) { P.st->vl_count[0] = 0; P.st->vl_count[1] = 0; }
-      g.sync();
-      // the removed vertices: from the list of every vertex sent back when
-      // few (and the sub-steps' classification did not reuse its buffer),
-      // else by a pass over the vertices
-      const bool from_list = few && !(nrev > 0 && P.substeps > 0);
-      const int nscan = from_list ? nall : P.V_it;
-      WarpBuf wins{warp_buf(0), 0};
-      for (int base = (from_list ? spread_tid() - (int)(threadIdx.x & 31) : blockIdx.x * blockDim.x); base < nscan;
-           base += stride) {
-        const int vi = base + (from_list ? (int)(threadIdx.x & 31) : (int)threadIdx.x);
-        const int v = vi < nscan ? (from_list ? ld_i(P.hard + vi) : vert_at(P, vi)) : 0;
+      WarpBuf wb{warp_buf(0), 0};
+      for (int base = blockIdx.x * blockDim.x; base < P.E_it; base += stride) {
+        const int ei = base + threadIdx.x;
+        const int e = ei < P.E_it ? edge_at(P, ei) : -1;
         int mine[1];
         int k = 0;
-        if (vi < nscan && ld_i(P.vhe + v) < 0 && marked(Q, v, fs)) {
-          __stcg(P.pos + v, __ldcg(P.target + v));
-          mine[k++] = v;
-        }
-        wb_push(wins, mine, k, P.vl0, &P.st->vl_count[0], P.V, P.st);
+        if (e >= 0 && (unsigned)ld_i(reinterpret_cast<const int*>(P.qmark) + e) == mk) mine[k++] = e;
+        if (__any_sync(kFull, k > 0)) wb_push(wb, mine, k, P.wl0, &P.st->wl_count[0], P.E, P.st);
       }
-      wb_flush(wins, P.vl0, &P.st->vl_count[0], P.V, P.st);
+      wb_flush(wb, P.wl0, &P.st->wl_count[0], P.E, P.st);
       g.sync();
-      if (ok) ok = phase_insert(g, Q, stamp, lc, mk);
-      g.sync();
+      phase_lawson<false>(g, Q, 0, stamp, lc, 0);
     } else {
-      timeline(P, 44);
-    }
-    timeline(P, 45);
-    // (4) one Lawson pass from every marked edge: work-list 0 holds the
-    // classification's non-Delaunay edges and the appended marks, repeats
-    // included; deduplicated into work-list 1 when short, else rebuilt from
-    // the marks over every edge
-    if (ok) {
-      const int nw = ld_i(&P.st->wl_count[0]);
-      const bool rebuild = ld_i(&P.st->mark_ovf) || (long long)nw * 4 >= (long long)P.E_it;
-      g.sync();  // every thread has read the count and the flag
-      if (rebuild) {
-        if (gtid == 0) { P.st->wl_count[0] = 0; P.st->wl_count[1] = 0; }
-        g.sync();
-        WarpBuf wb{warp_buf(0), 0};
-        for (int base = blockIdx.x * blockDim.x; base < P.E_it; base += stride) {
-          const int ei = base + threadIdx.x;
-          const int e = ei < P.E_it ? edge_at(P, ei) : -1;
-          int mine[1];
-          int k = 0;
-          if (e >= 0 && (unsigned)ld_i(reinterpret_cast<const int*>(P.qmark) + e) == mk) mine[k++] = e;
-          if (__any_sync(kFull, k > 0)) wb_push(wb, mine, k, P.wl0, &P.st->wl_count[0], P.E, P.st);
-        }
-        wb_flush(wb, P.wl0, &P.st->wl_count[0], P.E, P.st);
-        g.sync();
-        phase_lawson<false>(g, Q, 0, stamp, lc, 0);
-      } else {
-        const unsigned du = stamp++;  // first sight of an edge in this pass (cand is free until the flip rounds)
-        if (gtid == 0) P.st->wl_count[1] = 0;
-        g.sync();
-        WarpBuf wb{warp_buf(0), 0};
-        for (int base = spread_tid() - (int)(threadIdx.x & 31); base < nw; base += stride) {
-          const int i = base + (int)(threadIdx.x & 31);
-          int mine[1];
-          int k = 0;
-          if (i < nw) {
-            const int e = ld_i(P.wl0 + i);
-            if (e >= 0 && e < P.E && atomicMax(P.cand + e, du) < du) mine[k++] = e;
-          }
-          if (__any_sync(kFull, k > 0)) wb_push(wb, mine, k, P.wl1, &P.st->wl_count[1], P.E, P.st);
-        }
-        wb_flush(wb, P.wl1, &P.st->wl_count[1], P.E, P.st);
-        if (gtid == 0) P.st->wl_count[0] = 0;
-        g.sync();
-        phase_lawson<false>(g, Q, 1, stamp, lc, 0);
-      }
+      const unsigned du = stamp++;  // first sight of an edge in this pass (cand is free until the flip rounds)
+      if (gtid == 0) P.st->wl_count[1] = 0;
       g.sync();
+      WarpBuf wb{warp_buf(0), 0};
+      for (int base = spread_tid() - (int)(threadIdx.x & 31); base < nw; base += stride) {
+        const int i = base + (int)(threadIdx.x & 31);
+        int mine[1];
+        int k = 0;
+        if (i < nw) {
+          const int e = ld_i(P.wl0 + i);
+          if (e >= 0 && e < P.E && atomicMax(P.cand + e, du) < du) mine[k++] = e;
+        }
+        if (__any_sync(kFull, k > 0)) wb_push(wb, mine, k, P.wl1, &P.st->wl_count[1], P.E, P.st);
+      }
+      wb_flush(wb, P.wl1, &P.st->wl_count[1], P.E, P.st);
+      if (gtid == 0) P.st->wl_count[0] = 0;
+      g.sync();
+      phase_lawson<false>(g, Q, 1, stamp, lc, 0);
     }
-    timeline(P, 46);
+    g.sync();
   }
+  timeline(P, 46);
   flush_counters(P, lc);
   return stamp;
 }
@@ -2717,15 +2738,51 @@ __device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, 
   if (at < P.V) __stcg(list + at, u);
 }
 
-// A step that moved few vertices of a mesh larger than this is left to the removal
-// path, whose cost goes with the movers; the stars' goes with the mesh.
+// Stars or removal?  The stars' time goes with the mesh (every vertex is copied, checked
+// and written), removal's with the edges that are not Delaunay and the faces turned, in
+// rounds that a larger mesh fills better.  Removal goes first where
+//  - few vertices moved (`sparse`: only their stars were classified) and the mesh has
+//    more than kStarSparse vertices: 460,000 vertices of which 2 % move, stars 1117 us a
+//    pass, removal 800; 200,000 and below, stars 0.6 to 0.9 of removal at any number of
+//    movers;
+//  - the mesh has more than kStarMost vertices.  Uniform points, sigma = 0.1 x spacing,
+//    stars and removal in ms: 1M 1.23 and 1.67, 2M 2.12 and 2.15, 2.5M 2.58 and 2.48, 3M
+//    3.12 and 2.92, 4M 4.06 and 3.29, 8.5M 8.34 and 6.05;
+//  - between 670,000 and kStarMost vertices, when all move and few of the edges are open
+//    (not Delaunay).  Counted twice where hardly a face has turned, as then the stars
+//    agree after a round or two (a random walk), and as a third where most vertices
+//    stayed.  us by stars and by removal:
+//      vertices  open edges  turned   stars  removal
+//       700,000       3,400      50     477      390
+//       500,000       2,500      50     348      446
+//     1,000,000       4,800      40     580      489
+//     1,000,000      16,200   3,000    1056      829
+//     1,000,000     109,000  32,000    1400     1422
+//     1,000,000      22,900     150     734      932   a walk of 0.01 x spacing
+//     2,000,000      10,400     320     992      615
+//     2,000,000     119,600  31,000    1891     1407
+//     2,000,000     592,600 158,000    2454     2767   a walk of 0.15 x spacing
+//    Over 135 such steps of 500,000 to 2.5M vertices the rule's side is 0.3 % slower than
+//    the better one on average, 5 % slower than removal at most.
 constexpr int kStarSparse = 200000;
-
-// So is every step of a mesh larger than this: the stars' time goes with the vertices
-// (1.0 us a thousand), the removal path's rounds wait less per vertex the more they
-// hold.  Uniform points, sigma = 0.1 x spacing, stars and removal in ms: 1M 1.23 and
-// 1.72, 2M 2.11 and 2.35, 3M 3.12 and 2.92, 4M 4.06 and 3.29, 8.5M 8.34 and 6.05.
 constexpr int kStarMost = 2500000;
+constexpr int kStarDense = 850000;   // open edges allowed: 0.28 a vertex above this
+constexpr int kStarTurned = 670000;  // the least vertices where a handful of turned faces goes to removal
+__device__ __forceinline__ bool removal_first(const KParams& P, int turned, bool sparse) {
+  if (P.V_it > kStarMost || (sparse && P.V_it > kStarSparse)) return true;
+  if (P.V_it <= kStarTurned) return false;
+  const long long n = ld_i(&P.st->wl_count[0]);
+  if (turned < 128 && 128 * n < P.V_it) return true;
+  const long long movers = P.move_mode == MOVE_NONE ? P.V_it : ld_i(&P.st->movers_now);
+  const float open = 4 * movers < P.V_it ? 0.333f * (float)n : (32ll * turned < n ? 2.f : 1.f) * (float)n;
+  return open < 0.28f * (float)(P.V_it - kStarDense);
+}
+// Removal is given up for stars while vertices are still being sent back, when they are
+// more than twice the turned faces' sides and this: where neighbours move together, far
+// beyond their spacing, each vertex sent back turns the next face over until most of the
+// mesh is on its way back (20,000 points in a Taylor-Green flow, three spacings a step:
+// one face turned, 16,000 vertices; from 100,000 points the send-back did not end).
+constexpr int kSentBack = 1024;
 
 // The vertices of the block's run marked with cs, in order, onto a list.
 __device__ __forceinline__ void star_marked(const KParams& P, unsigned cs, int i0, int i1, int* list, int* count) {
@@ -2755,6 +2812,8 @@ constexpr int kWarpStars = 8;
 // two barriers later, so all take the same branches; bit 30 of the next count says
 // that a star could not be made.
 // kBuild: there is no mesh yet, the first stars come from the Morton order.
+// A vertex that this launch has marked (from q0 on: by the classification, or by a
+// send-back given up) makes its first star anew, any other keeps its ring.
 template <bool kBuild>
 __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, unsigned& stamp, unsigned q0,
                                           unsigned sc0, LocalCounters& lc) {
@@ -2778,7 +2837,7 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
     for (int i = i0 + warp; i < i1; i += kThreads / 32) {
       const int v = vert_at(P, i);
       if (P.vfix[v]) continue;
-      const bool keep = (unsigned)ld_i(P.vmark + v) != q0;
+      const bool keep = (unsigned)ld_i(P.vmark + v) < q0;
       if (lane == 0) made += keep ? 0 : 1;
       if (!warp_from_mesh(P, v, keep, sc0, lc) && lane == 0) fine = star_alone(P, v, keep, sc0, false, lc) && fine;
       __syncwarp();
@@ -2786,7 +2845,7 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
   } else {
     for (int base = i0 + warp * 32; base < i1; base += kThreads) {
       const int v = base + lane < i1 ? vert_at(P, base + lane) : -1;
-      const bool keep = v >= 0 && (unsigned)ld_i(P.vmark + v) != q0;
+      const bool keep = v >= 0 && (unsigned)ld_i(P.vmark + v) < q0;
       int rc = kStarOk;
       if (v >= 0 && !P.vfix[v]) {
         SharedCand L;
@@ -2930,14 +2989,13 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
       cs = stamp++;
       int* next = lists[slot & 1];
       int* count = cnt + slot % 3;
-      // before anything joins (and of one mind with the blocks that already add to it):
-      // an append to a count that holds the bit is taken for a list that is full, an
-      // error of the step
-      if (ld_i(count) & kStarGivenUp) return false;
       if (gtid == 0) cnt[(slot + 1) % 3] = 0;
       int inner;
       unsigned long long ranks;
       if (many) {
+        // before anything joins: an append to a count that holds the bit is taken for a
+        // list that is full, an error of the step (star_list leaves such an entry out)
+        if (ld_i(count) & kStarGivenUp) return false;
         auto again = [&](int u) { __stcg(P.smark + u, cs); };
         for (int i = spread_tid(); i < n; i += stride) {
           const int v = ld_i(list + i);
@@ -2956,6 +3014,7 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
       }
       g.sync();
       n = ld_i(count);
+      if (n >= kStarGivenUp) return false;
       if (n == 0) ++slot;
     }
     touched = all_few ? ts : 0;
@@ -2992,7 +3051,6 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
     if (!(few ? warp_commit(P, v) : star_commit(P, v))) set_error(P, MCL_ERR_DEGENERATE_INPUT);
   }
   if (gtid == 0) {
-    P.st->c[C_INVERTED] += (unsigned long long)ld_i(&P.st->inverted);
     const unsigned long long m = (unsigned long long)ld_i(&P.st->star_made);
     P.st->c[C_REVERTED] += m;
     P.st->c[C_REMOVED] += m;
@@ -3011,15 +3069,39 @@ __global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KP
   unsigned stamp = ld_i(reinterpret_cast<const int*>(&P.st->epoch));
   timeline(P, 0);
   const unsigned q0 = stamp++;
+  __shared__ unsigned s_q0;
+  if (threadIdx.x == 0) s_q0 = q0;
   const unsigned sc0 = stamp++;
   const bool sparse = phase_classify<true>(g, P, q0, sc0, lc);
   g.sync();
   phase_classify_hard<true>(g, P, q0, sc0, lc);
   timeline(P, 1);
   const int inverted = ld_i(&P.st->inverted);
-  if (inverted == 0) phase_lawson<true, true>(g, P, 0, stamp, lc, sc0);
-  else if (P.substeps > 0 || !P.square || P.V_it > kStarMost || (sparse && P.V_it > kStarSparse) || !star_step<false>(g, P, stamp, q0, sc0, lc))
-    stamp = repair_step(g, P, stamp, q0);
+  if (inverted == 0) {
+    phase_lawson<true, true>(g, P, 0, stamp, lc, sc0);
+  } else {
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (first) P.st->c[C_INVERTED] += (unsigned long long)inverted;
+    // no stars where sub-steps are asked for, and on a mesh that is not its square's
+    const bool never = P.substeps > 0 || !P.square;
+    const unsigned fs = stamp++;
+    int rc = kSentBackMany;
+    if (never || removal_first(P, inverted, sparse))
+      rc = send_back(g, P, fs, never ? LLONG_MAX : 2ll * inverted + kSentBack);
+    if (rc == MCL_OK || never) {
+      if (rc == MCL_OK) stamp = repair_step(g, P, stamp, q0, fs);
+      else if (first) set_error(P, rc);
+    } else {
+      // Nothing lives over the send-back's call that the stars need: the counters are
+      // flushed and the stamps read again, which keeps registers for the loops of
+      // star_step (1M random walkers 1265 -> 1245 us).
+      flush_counters(P, lc);
+      lc = LocalCounters{0, 0, 0, 0, 0, 0, 0};
+      const unsigned q = s_q0;
+      stamp = q + 3;  // q, q + 1 and fs are taken
+      if (!star_step<false>(g, P, stamp, q, q + 1, lc)) stamp = repair_step(g, P, stamp, q, 0);
+    }
+  }
   flush_counters(P, lc);
   // No closing grid barrier: each block leaves when its own work is done and
   // the last one to leave publishes the launch.  The block barrier orders its

@@ -1,0 +1,94 @@
+"""Which way a step with turned faces goes: stars (no edge is flipped), removal and
+reinsertion, removal after stars that could not be made, and stars after a send-back
+that took most of the mesh.  Every mesh equals the oracle's exact triangulation."""
+import numpy as np
+import pytest
+
+from helpers import gaussian_disp, spacing, uniform_points
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def M():
+    import torch
+
+    import mcleap_gb300 as M
+    from mcleap_gb300 import build as B
+
+    assert torch.cuda.is_available()
+    B.build()
+    M.lib()
+    return M
+
+
+def step(b, pos, d, meshes=(0,)):
+    """One step of the batch; checks it against the oracle and returns (stats, positions)."""
+    import torch
+
+    st = b.step(torch.from_numpy(np.ascontiguousarray(d, np.float32)).cuda())
+    assert st["status"] == 0, st
+    assert not b.validate().any()
+    pos = (pos + d).astype(np.float32)
+    for i in meshes:
+        v0, nv = int(b.v0[i]), int(b.nv[i])
+        assert np.array_equal(b.download(i)[0], pos[v0:v0 + nv])
+        assert np.array_equal(b.edges(i), O.Mesh.build(pos[v0 + 4:v0 + nv], exact=True).edges())
+    return st, pos
+
+
+def positions(b):
+    return np.concatenate([b.download(i)[0] for i in range(b.count)])
+
+
+@pytest.mark.parametrize("tile", [0, 1, 32])
+def test_few_movers_of_a_large_mesh(M, tile):
+    """Above 200,000 vertices steps that move few of them go by removal; the mesh beside
+    it is active in every other step."""
+    b = M.MeshBatch.from_points([uniform_points(200500, 1), uniform_points(3000, 2)])
+    b.set_tuning(removal_tile=tile)
+    pos = positions(b)
+    rng = np.random.default_rng(tile)
+    for k in range(4):
+        b.set_active([0] if k % 2 else None)
+        d = np.zeros_like(pos)
+        m = rng.integers(4, b.nv[0], 2000)
+        d[m] = rng.standard_normal((2000, 2)) * 0.5 * spacing(200500)
+        if k % 2 == 0:
+            m = rng.integers(b.v0[1] + 4, b.V, 30)
+            d[m] = rng.standard_normal((30, 2)) * 0.5 * spacing(3000)
+        d[(pos + d < 0).any(1) | (pos + d >= 8192).any(1)] = 0
+        st, pos = step(b, pos, d, (0, 1))
+        assert st["inverted_faces"] > 0
+        # the first step classifies every edge: whether few move is known from the last
+        if k:
+            assert st["lawson_flips"] > 0 and st["insert_rounds"] > 0
+    b.close()
+
+
+def test_few_turned_faces_of_a_large_mesh(M):
+    """From 850,000 vertices on few open edges go by removal, many by stars."""
+    n = 900000
+    b = M.MeshBatch.from_points([uniform_points(n, 3)])
+    pos = positions(b)
+    st, pos = step(b, pos, gaussian_disp(b.V, 0.001 * spacing(n), 1, clamp_pos=pos))
+    assert st["inverted_faces"] > 0 and st["lawson_flips"] > 0
+    st, pos = step(b, pos, gaussian_disp(b.V, 0.1 * spacing(n), 2, clamp_pos=pos))
+    assert st["inverted_faces"] > 0 and st["lawson_flips"] == 0
+    b.close()
+
+
+@pytest.mark.parametrize("n,far", [(900000, 3.0)])
+def test_neighbours_that_move_together_far(M, n, far):
+    """A swirl of several spacings a step turns few faces; sending their vertices back
+    would send back their neighbours in turn."""
+    b = M.MeshBatch.from_points([uniform_points(n, 4)])
+    pos = positions(b)
+    for k in range(2):
+        u = (pos.astype(np.float64) / 8192 * 6.2 + 0.04) * (1 + 0.001 * k)
+        d = np.stack([np.sin(u[:, 0]) * np.cos(u[:, 1]), -np.cos(u[:, 0]) * np.sin(u[:, 1])], 1) * far * spacing(n)
+        d[:4] = 0
+        st, pos = step(b, pos, d.astype(np.float32))
+        assert st["inverted_faces"] > 0 and st["lawson_flips"] == 0, st
+    b.close()
