@@ -1863,6 +1863,7 @@ __device__ void finish_launch(const KParams& P, unsigned stamp) {
   }
   const unsigned long long tm = __ldcg(&st->tsmax[lane & 3]);
   const int status = __ldcg(&st->status), site = __ldcg(&st->site), movers = __ldcg(&st->movers_now);
+  const int tried = __ldcg(&st->star_tried), fails = __ldcg(&st->star_fails), hold = __ldcg(&st->star_hold);
   const unsigned long long calls = __ldcg(&st->calls), failed = __ldcg(&st->failed);
   if (lane < C_COUNT) {
     st->last[lane] = c;
@@ -1895,6 +1896,19 @@ __device__ void finish_launch(const KParams& P, unsigned stamp) {
   for (int i = 0; i < 3; ++i) st->star_n[i] = 0;
   st->star_ext = 0;
   st->star_made = 0;
+  // Stars that could not be made (one wider than 128, more wide ones than rows) are left
+  // out of the next steps, twice as many each time, 32 at most: such a mesh paid for them
+  // and for removal on every step (one vertex of 150 neighbours among 1,000,000: 1650 us
+  // by removal alone, 2310 with both).
+  if (tried == kStarsMade) {
+    st->star_hold = st->star_fails = 0;
+  } else if (tried == kStarsFailed) {
+    st->star_fails = min(fails + 1, 5);
+    st->star_hold = 1 << min(fails + 1, 5);
+  } else if (tried == kStarsHeld) {
+    st->star_hold = hold - 1;
+  }
+  st->star_tried = 0;
   st->fix_all = 0;
   st->mark_ovf = 0;
   st->movers_last = movers;
@@ -3076,19 +3090,21 @@ __global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KP
   g.sync();
   phase_classify_hard<true>(g, P, q0, sc0, lc);
   timeline(P, 1);
-  const int inverted = ld_i(&P.st->inverted);
+  const int inverted = ld_i(&P.st->inverted), hold = ld_i(&P.st->star_hold);
   if (inverted == 0) {
     phase_lawson<true, true>(g, P, 0, stamp, lc, sc0);
   } else {
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
     if (first) P.st->c[C_INVERTED] += (unsigned long long)inverted;
-    // no stars where sub-steps are asked for, and on a mesh that is not its square's
-    const bool never = P.substeps > 0 || !P.square;
+    // no stars where sub-steps are asked for, on a mesh that is not its square's, and for
+    // a while after they could not be made
+    const bool never = P.substeps > 0 || !P.square, held = hold > 0;
     const unsigned fs = stamp++;
     int rc = kSentBackMany;
-    if (never || removal_first(P, inverted, sparse))
+    if (never || held || removal_first(P, inverted, sparse))
       rc = send_back(g, P, fs, never ? LLONG_MAX : 2ll * inverted + kSentBack);
     if (rc == MCL_OK || never) {
+      if (first && held) P.st->star_tried = kStarsHeld;
       if (rc == MCL_OK) stamp = repair_step(g, P, stamp, q0, fs);
       else if (first) set_error(P, rc);
     } else {
@@ -3099,7 +3115,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KP
       lc = LocalCounters{0, 0, 0, 0, 0, 0, 0};
       const unsigned q = s_q0;
       stamp = q + 3;  // q, q + 1 and fs are taken
-      if (!star_step<false>(g, P, stamp, q, q + 1, lc)) stamp = repair_step(g, P, stamp, q, 0);
+      const bool done = star_step<false>(g, P, stamp, q, q + 1, lc);
+      if (blockIdx.x == 0 && threadIdx.x == 0) P.st->star_tried = done ? kStarsMade : kStarsFailed;
+      if (!done) stamp = repair_step(g, P, stamp, q, 0);
     }
   }
   flush_counters(P, lc);

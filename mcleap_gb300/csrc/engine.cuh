@@ -55,6 +55,8 @@ enum Counter {
 
 constexpr int kTimeline = 48;
 
+enum : int { kStarsMade = 1, kStarsFailed, kStarsHeld };
+
 constexpr float kSquare = 10000000.0f;  // the bounding square's corners are at +-this
 
 struct DevState {
@@ -75,6 +77,7 @@ struct DevState {
   int star_n[3];           // vertices whose stars disagree, per round (triple-buffered; bit 30: given up)
   int star_ext;            // overflow rows taken by this launch
   int star_made;           // stars made anew by this launch
+  int star_tried;          // this launch's untangling by stars (kStarsMade and the others; 0: none)
   int sub_count[3];        // repair sub-steps: mover lists (2), vertices left for removal
   int sub_rev[3];          // movers sent back per sub-step pass (triple-buffered)
   unsigned int epoch;      // next unused stamp
@@ -82,6 +85,10 @@ struct DevState {
   unsigned int arrived;    // blocks of k_step that have finished (the last one publishes)
   unsigned int stamp_max;  // largest next-free stamp over those blocks
   unsigned long long c[C_COUNT];
+  // kept between launches: how many more launches leave stars out, and how often in a row
+  // they could not be made
+  int star_hold;
+  int star_fails;
   // published by the last launch
   int last_status;
   int last_site;

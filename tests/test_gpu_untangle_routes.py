@@ -42,6 +42,47 @@ def positions(b):
     return np.concatenate([b.download(i)[0] for i in range(b.count)])
 
 
+@pytest.mark.parametrize("spokes", [127, 128, 129, 150])
+def test_a_star_wider_than_the_lists(M, spokes):
+    """A hub that stars have no room for, from 129 spokes on: each step goes by removal, the
+    two after the first without trying stars (which test a circle for each vertex at
+    least), and stars come back, within as many steps as they were left out for, once the
+    hub has closed."""
+    c = np.array([4096.0, 4096.0])
+    p = uniform_points(3000, spokes)
+    p = p[np.hypot(*(p - c).T) > 700]
+    a = np.linspace(0, 2 * np.pi, spokes, endpoint=False) + 0.1
+    p = np.concatenate([p, c[None], c + 600 * np.stack([np.cos(a), np.sin(a)], 1)]).astype(np.float32)
+    b = M.MeshBatch.from_points([p])
+    pos = positions(b)
+    near = np.hypot(*(pos - c).T) < 650
+    rng = np.random.default_rng(spokes)
+    walk = gaussian_disp(b.V, 0.3 * spacing(3000), spokes, clamp_pos=pos)
+    walk[np.hypot(*(pos - c).T) < 1000] = 0
+    back = (pos - (pos + walk).astype(np.float32)).astype(np.float32)
+    tests = []
+    for k in range(9):  # there and back
+        st, pos = step(b, pos, back if k % 2 else walk)
+        assert st["inverted_faces"] > 0
+        widest = np.bincount(b.edges(0).ravel()).max()
+        assert widest >= spokes
+        assert st["lawson_flips"] > 0 or widest <= 128
+        tests.append(st["incircle_tests"])
+    if spokes > 128:
+        made = np.count_nonzero(walk.any(1))
+        assert tests[2] + made // 2 < tests[0], tests
+    d = np.zeros_like(pos)
+    rim = near & (np.hypot(*(pos - c).T) > 1)
+    d[rim] = rng.standard_normal((rim.sum(), 2)) * 40
+    st, pos = step(b, pos, d)
+    by_stars = []
+    for k in range(9):
+        st, pos = step(b, pos, gaussian_disp(b.V, 0.3 * spacing(3000), 71 * k + spokes, clamp_pos=pos))
+        by_stars.append(st["lawson_flips"] == 0)
+    assert by_stars[-1]
+    b.close()
+
+
 @pytest.mark.parametrize("tile", [0, 1, 32])
 def test_few_movers_of_a_large_mesh(M, tile):
     """Above 200,000 vertices steps that move few of them go by removal; the mesh beside
