@@ -71,10 +71,14 @@ constexpr int kMaxDeg = 4096;
 // while it is in flight (CountSlot).  Each thread says whether its own query counts, a
 // block adds once (500,000 rows all cut off and added one by one: 350 us).  A call that
 // asks for no count passes no cell.
-__device__ __forceinline__ void count_done(bool mine, unsigned long long* cell, unsigned long long* host) {
+// count_add: of a kernel that another one of the same call follows.
+__device__ __forceinline__ void count_add(bool mine, unsigned long long* cell) {
   const int all = __syncthreads_count(mine);
+  if (threadIdx.x == 0 && all) atomicAdd(cell, (unsigned long long)all);
+}
+__device__ __forceinline__ void count_done(bool mine, unsigned long long* cell, unsigned long long* host) {
+  count_add(mine, cell);
   if (threadIdx.x == 0) {
-    if (all) atomicAdd(cell, (unsigned long long)all);
     __threadfence();
     if (atomicAdd(cell + 1, 1ull) == gridDim.x - 1) {
       __threadfence();
@@ -310,13 +314,13 @@ __global__ void k_closest(const float2* pos, int V, int layout, int max_ring, co
 // include/kernels.cuh:169-219); the found set is written sorted ascending.
 constexpr int kFrnnLocal = 256;
 
-// One thread's search, depth first, for sets that a warp's lists do not hold:
+// One thread's search, in the order found, for sets that a part's lists do not hold:
 // up to kFrnnLocal vertices, in a thread-local list.  Writes the row; returns whether it
 // or the list was too short.
 __device__ __noinline__ bool frnn_serial(const MeshView M, int i, float r2, int cap, size_t stride, int* row) {
   int found[kFrnnLocal];
   int nf = 0;
-  int top = 0;  // stack = found[top..nf): vertices whose rings are still to scan
+  int top = 0;  // found[top..nf): vertices whose rings are still to scan
   bool over = false;
   const float2 pi = M.pos[i];
   int cur = i;
@@ -327,10 +331,9 @@ __device__ __noinline__ bool frnn_serial(const MeshView M, int i, float r2, int 
       do {
         const int w = mv_origin(M, h ^ 1);
         if (w != i) {
-          bool seen = false;
-          for (int k = 0; k < nf; ++k)
-            if (found[k] == w) { seen = true; break; }
-          if (!seen && sqdist(pi, M.pos[w]) <= r2) {
+          bool seen = sqdist(pi, M.pos[w]) > r2;
+          for (int k = 0; k < nf && !seen; ++k) seen = found[k] == w;
+          if (!seen) {
             if (nf < kFrnnLocal) found[nf++] = w;
             else over = true;
           }
@@ -354,35 +357,36 @@ __device__ __noinline__ bool frnn_serial(const MeshView M, int i, float r2, int 
   return over || nf > cap;
 }
 
-// Half a warp's search, breadth first: two lanes walk the ring of one vertex of the
-// frontier from its first spoke, one each way, until they meet; a lane's neighbour
-// within r joins through a hash set in shared memory.  The search is a chain of
+// The search of kLanes lanes (half a warp), breadth first: two lanes walk the ring of one
+// vertex of the frontier from its first spoke, one each way, until they meet; a lane's
+// neighbour within r joins through a hash set in shared memory.  The search is a chain of
 // dependent loads, so the time is the number of steps one after another: about
 // four a level for a ring of six, three or four levels for r = 2 x spacing, where a
 // thread alone takes a step for each of some eighty spokes and looks each up in its
 // own list in local memory.  With a warp to a query 13 of its lanes had work and it was
 // bound by instruction issue (2600 a query); a frontier is seldom wider than the eight
 // vertices that half a warp takes at once.  60,000 queries, r = 2 x spacing, GB300:
-// 567 us by threads, 168 us by warps; the served list 163 us by warps, 120 by half warps (127 by quarters).
+// 567 us by threads, 168 us by warps; the served list 163 us by warps, 120 by half warps
+// (127 by quarters).
 constexpr int kFrnnWarps = 4;
 constexpr int kFrnnFound = 64;
 constexpr int kFrnnHash = 128;
 
-// Both halves of a warp call it together; a half with no query has i = -1.  Returns
-// false in a half that found more than its list holds.
-constexpr int kFrnnLanes = 16;
-__device__ __forceinline__ bool half_search(const MeshView& M, int i, float r2, int* found, int* hash, int* count) {
-  const int lane = threadIdx.x & 31, sub = lane & (kFrnnLanes - 1), way = lane & 1;
-  const unsigned half = ((1u << kFrnnLanes) - 1u) << (lane - sub), lt = half & ((1u << lane) - 1u);
+// All parts of a warp call it together; a part with no query has i = -1.  Returns
+// false in a part that found more than its list holds.
+template <int kLanes>
+__device__ __forceinline__ bool part_search(const MeshView& M, int i, float r2, int* found, int* hash, int* count) {
+  const int lane = threadIdx.x & 31, sub = lane & (kLanes - 1), way = lane & 1;
+  const unsigned part = ((1u << kLanes) - 1u) << (lane - sub), lt = part & ((1u << lane) - 1u);
 #pragma unroll
-  for (int k = 0; k < kFrnnHash / kFrnnLanes; ++k) hash[kFrnnLanes * k + sub] = -1;
+  for (int k = 0; k < kFrnnHash / kLanes; ++k) hash[kLanes * k + sub] = -1;
   __syncwarp();
   bool live = i >= 0, fits = true;
   const float2 pi = live ? M.pos[i] : make_float2(0.f, 0.f);
   int nf = 0, lo = -1;  // the frontier: i, then found[lo .. hi)
   while (__any_sync(0xffffffffu, live && lo < nf)) {
     const int hi = lo < 0 ? 0 : nf;
-    for (int c = lo; __any_sync(0xffffffffu, live && c < hi); c += kFrnnLanes / 2) {
+    for (int c = lo; __any_sync(0xffffffffu, live && c < hi); c += kLanes / 2) {
       const int j = c + (sub >> 1);
       const int u = !live || c >= hi ? -1 : (lo < 0 ? (j == lo ? i : -1) : (j < hi ? found[j] : -1));
       const int h0 = u >= 0 ? __ldg(M.vhe + u) : -1;
@@ -409,7 +413,7 @@ __device__ __forceinline__ bool half_search(const MeshView& M, int i, float r2, 
             k = (k + 1) & (kFrnnHash - 1);
           }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, fresh) & half;
+        const unsigned m = __ballot_sync(0xffffffffu, fresh) & part;
         if (fresh) {
           const int at = nf + __popc(m & lt);
           if (at < kFrnnFound) found[at] = w;
@@ -434,36 +438,60 @@ __device__ __forceinline__ bool half_search(const MeshView& M, int i, float r2, 
   return fits;
 }
 
-// Rows for the vertices verts[0 .. n) (NULL: all of them), half a warp each.  With
+// Rows for the vertices verts[0 .. n) (NULL: all of them), kLanes lanes each.  With
 // rcomp the radius of vertex i is rcomp[vcomp[i]] (one radius per mesh of a batch; a
 // plain mesh has vcomp == nullptr and one radius).
-__global__ void __launch_bounds__(32 * kFrnnWarps) k_mesh_frnn(MeshView M, const int* verts, int n, float r2,
-                                                               int layout, int max_frnn, int* out,
-                                                               unsigned long long* cell,
-                                                               unsigned long long* host, const float* rcomp,
-                                                               const int* vcomp) {
-  constexpr int kPer = 32 / kFrnnLanes * kFrnnWarps;  // queries per block
+//
+// Sets that the lists do not hold are one thread's work.  Up to kFrnnFew queries the
+// part's first lane does it; of more they are left, marked by a count of kFrnnLeft, to
+// k_mesh_frnn_left, a thread each: one lane in sixteen at work is bound by instruction
+// issue (78 neighbours each: 200,000 queries 66 ms by first lanes, 9.9 by threads; 20,000:
+// 8.4 and 2.5; 1,000: 1.1 and 2.8).
+struct FrnnQuery {
+  const int* verts;
+  int n;
+  float r2;
+  int layout, max_frnn;
+  int* out;
+  const float* rcomp;
+  const int* vcomp;
+
+  __device__ __forceinline__ int vertex(const MeshView& M, int q) const {
+    const int i = q < n ? (verts ? __ldg(verts + q) : q) : -1;
+    return i >= M.V || (i >= 0 && __ldg(M.vhe + i) < 0) ? -1 : i;
+  }
+  __device__ __forceinline__ float radius2(int i) const {
+    if (!rcomp || i < 0) return r2;
+    const float rc = rcomp[vcomp ? vcomp[i] : 0];
+    return __fmul_rn(rc, rc);
+  }
+  __device__ __forceinline__ int* row(int q) const {
+    return layout == MCL_LAYOUT_COLUMN ? out + q : out + (size_t)q * max_frnn;
+  }
+  __device__ __forceinline__ size_t stride() const { return layout == MCL_LAYOUT_COLUMN ? (size_t)n : 1; }
+};
+constexpr int kFrnnFew = 2048;
+constexpr int kFrnnLeft = -1;
+
+template <int kLanes>
+__global__ void __launch_bounds__(32 * kFrnnWarps) k_mesh_frnn(MeshView M, FrnnQuery Q, unsigned long long* cell,
+                                                               unsigned long long* host) {
+  constexpr int kPer = 32 / kLanes * kFrnnWarps;  // queries per block
   __shared__ int found_s[kPer][kFrnnFound];
   __shared__ int hash_s[kPer][kFrnnHash];
-  const int sub = threadIdx.x & (kFrnnLanes - 1), slot = threadIdx.x / kFrnnLanes;
-  const int q = blockIdx.x * kPer + slot;
-  int i = q < n ? (verts ? __ldg(verts + q) : q) : -1;
-  const int cap = max_frnn - 1;
-  int* row = layout == MCL_LAYOUT_COLUMN ? out + q : out + (size_t)q * max_frnn;
-  const size_t stride = layout == MCL_LAYOUT_COLUMN ? (size_t)n : 1;
-  if (i >= M.V || (i >= 0 && __ldg(M.vhe + i) < 0)) i = -1;
-  if (q < n && i < 0 && sub == 0) row[0] = 0;
-  if (rcomp && i >= 0) {
-    const float rc = rcomp[vcomp ? vcomp[i] : 0];
-    r2 = __fmul_rn(rc, rc);
-  }
+  const int sub = threadIdx.x & (kLanes - 1), slot = threadIdx.x / kLanes;
+  const int q = blockIdx.x * kPer + slot, i = Q.vertex(M, q), cap = Q.max_frnn - 1;
+  int* row = Q.row(q);
+  const size_t stride = Q.stride();
+  if (q < Q.n && i < 0 && sub == 0) row[0] = 0;
+  const float r2 = Q.radius2(i);
   const int* found = found_s[slot];
   int nf = 0;
-  const bool fits = half_search(M, i, r2, found_s[slot], hash_s[slot], &nf);
+  const bool fits = part_search<kLanes>(M, i, r2, found_s[slot], hash_s[slot], &nf);
   bool cut = false;
   __syncwarp();
   if (i >= 0 && fits) {
-    for (int k = sub; k < nf; k += kFrnnLanes) {
+    for (int k = sub; k < nf; k += kLanes) {
       const int x = found[k];
       int rank = 0;
       for (int j = 0; j < nf; ++j) rank += found[j] < x ? 1 : 0;
@@ -474,7 +502,136 @@ __global__ void __launch_bounds__(32 * kFrnnWarps) k_mesh_frnn(MeshView M, const
       cut = nf > cap;
     }
   } else if (i >= 0 && sub == 0) {
-    cut = frnn_serial(M, i, r2, cap, stride, row);
+    if (Q.n > kFrnnFew) row[0] = kFrnnLeft;
+    else cut = frnn_serial(M, i, r2, cap, stride, row);
+  }
+  if (Q.n > kFrnnFew) {
+    if (host) count_add(cut, cell);
+  } else if (host) {
+    count_done(cut, cell, host);
+  }
+}
+
+// The same for more than kFrnnMany queries, whose time is the work: small sets are a
+// thread's own (up to kFrnnThread found, in its column of shared memory, and no more than
+// kFrnnRing of them beside i: more promise many), the others of the warp's 32 queries are
+// taken by its parts of kLanes lanes, as many at a time as there are.  us by threads
+// alone, by half warps alone, and by the form that the number of queries selects:
+//   queries    r / spacing  threads  halves     now
+//      60,000     0.3            42      44      44
+//                 2             343      95      94
+//     100,000     0.3            41      63      47
+//                 2             442     135     125
+//     200,000     0.3            43      98      43
+//                 2             610     247     348
+//                 5          10,770  66,300   9,860
+//   1,000,000     0.3           104     475     119
+//                 1             353     743     353
+//                 2           1,755   1,173   1,394
+//                 5          45,700     (*)  41,100
+// (*) a lone lane in sixteen for sets of more than 64.
+constexpr int kFrnnQuarters = 65536;  // quarter warps from here on, ...
+constexpr int kFrnnMany = 100000;     // ... and threads first
+constexpr int kFrnnThread = 12;
+constexpr int kFrnnRing = 4;
+template <int kLanes>
+__global__ void __launch_bounds__(32 * kFrnnWarps) k_mesh_frnn_many(MeshView M, FrnnQuery Q, unsigned long long* cell,
+                                                                    unsigned long long* host) {
+  constexpr int kParts = 32 / kLanes;
+  __shared__ int pool[kFrnnWarps][kParts * (kFrnnFound + kFrnnHash)];
+  static_assert(kParts * (kFrnnFound + kFrnnHash) >= 32 * kFrnnThread, "the threads' columns fit the parts' lists");
+  const int lane = threadIdx.x & 31, sub = lane & (kLanes - 1), part = lane / kLanes, cap = Q.max_frnn - 1;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, q0 = q - lane;
+  const int i = Q.vertex(M, q);
+  const size_t stride = Q.stride();
+  const float r2 = Q.radius2(i);
+  int* mine = pool[threadIdx.x >> 5];
+  int* col = mine + lane;
+  int nf = 0, cut = 0;
+  bool many = false;
+  if (i >= 0) {
+    const float2 pi = M.pos[i];
+    int top = 0, cur = i;
+    while (!many) {
+      const int h0 = __ldg(M.vhe + cur);
+      int h = h0, deg = 0;
+      if (h0 >= 0) {
+        do {
+          const int w = mv_origin(M, h ^ 1);
+          if (w != i && sqdist(pi, M.pos[w]) <= r2) {
+            bool seen = false;
+            for (int k = 0; k < nf && !seen; ++k) seen = col[32 * k] == w;
+            if (!seen) {
+              many = nf == (cur == i ? kFrnnRing : kFrnnThread);
+              if (many) break;
+              col[32 * nf++] = w;
+            }
+          }
+          h = mv_rot(M, h);
+          ++deg;
+        } while (h != h0 && deg < kMaxDeg);
+      }
+      if (top >= nf) break;
+      cur = col[32 * top++];
+    }
+  }
+  if (q < Q.n && !many) {
+    for (int a = 1; a < nf; ++a) {
+      const int x = col[32 * a];
+      int b = a - 1;
+      while (b >= 0 && col[32 * b] > x) { col[32 * (b + 1)] = col[32 * b]; --b; }
+      col[32 * (b + 1)] = x;
+    }
+    int* row = Q.row(q);
+    const int cnt = nf < cap ? nf : cap;
+    for (int k = 0; k < cnt; ++k) row[(size_t)(k + 1) * stride] = col[32 * k];
+    row[0] = cnt;
+    cut = nf > cap;
+  }
+  __syncwarp();
+  int* found = mine + part * (kFrnnFound + kFrnnHash);
+  for (unsigned todo = __ballot_sync(0xffffffffu, many); todo;) {
+    unsigned rest = todo;
+    for (int p = 0; p < part; ++p) rest &= rest - 1u;
+    const int src = rest ? __ffs((int)rest) - 1 : lane;
+    const int u = __shfl_sync(0xffffffffu, i, src);
+    const float ru = __shfl_sync(0xffffffffu, r2, src);
+    int got = 0;
+    const bool fits = part_search<kLanes>(M, rest ? u : -1, ru, found, found + kFrnnFound, &got);
+    __syncwarp();
+    if (rest) {
+      int* row = Q.row(q0 + src);
+      if (fits) {
+        for (int k = sub; k < got; k += kLanes) {
+          const int x = found[k];
+          int rank = 0;
+          for (int j = 0; j < got; ++j) rank += found[j] < x ? 1 : 0;
+          if (rank < cap) row[(size_t)(rank + 1) * stride] = x;
+        }
+      }
+      if (sub == 0) {
+        row[0] = !fits ? kFrnnLeft : (got < cap ? got : cap);
+        cut += fits && got > cap ? 1 : 0;
+      }
+    }
+    for (int p = 0; p < kParts; ++p) todo &= todo - 1u;
+    __syncwarp();
+  }
+  if (!host) return;
+  cut = __reduce_add_sync(0xffffffffu, cut);
+  if (lane == 0 && cut) atomicAdd(cell, (unsigned long long)cut);
+}
+
+__global__ void __launch_bounds__(128) k_mesh_frnn_left(MeshView M, FrnnQuery Q, unsigned long long* cell,
+                                                        unsigned long long* host) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  bool cut = false;
+  if (q < Q.n) {
+    int* row = Q.row(q);
+    if (row[0] == kFrnnLeft) {
+      const int i = Q.vertex(M, q);
+      cut = frnn_serial(M, i, Q.radius2(i), Q.max_frnn - 1, Q.stride(), row);
+    }
   }
   if (host) count_done(cut, cell, host);
 }
@@ -1128,10 +1285,14 @@ int launch_mesh_frnn(mcl_mesh* m, const int* verts, int64_t n, float r2, const f
     if (overflow) *overflow = 0;
     return MCL_OK;
   }
-  constexpr int kPer = 32 / kFrnnLanes * kFrnnWarps;
+  const FrnnQuery Q = {verts, (int)n, r2, layout, max_frnn, out, rcomp, rcomp ? m->vcomp : nullptr};
+  constexpr int kThreads = 32 * kFrnnWarps;
+  const int per = n <= kFrnnQuarters ? kThreads / 16 : n <= kFrnnMany ? kThreads / 8 : kThreads;  // queries per block
+  auto kernel = n <= kFrnnQuarters ? k_mesh_frnn<16> : n <= kFrnnMany ? k_mesh_frnn<8> : k_mesh_frnn_many<16>;
   return counted(m, s, overflow, [&](unsigned long long* cell, unsigned long long* host) {
-    k_mesh_frnn<<<(unsigned)((n + kPer - 1) / kPer), 32 * kFrnnWarps, 0, s>>>(
-        mesh_view(m), verts, (int)n, r2, layout, max_frnn, out, cell, host, rcomp, rcomp ? m->vcomp : nullptr);
+    kernel<<<(unsigned)((n + per - 1) / per), kThreads, 0, s>>>(mesh_view(m), Q, cell, host);
+    if (n > kFrnnFew)
+      k_mesh_frnn_left<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(mesh_view(m), Q, cell, host);
   });
 }
 
