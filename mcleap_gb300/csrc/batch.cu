@@ -145,8 +145,8 @@ __global__ void k_advance(unsigned long long* counter, int n, const int* act, in
 // alone (4 bytes, four slots per vertex, emptied before the call), so an insertion
 // is one compare-and-swap; with stamped entries that are never cleared it was a read
 // and a swap, after a pass that looked for meshes with movers, with the static
-// vertices inserted too (1M movers 160 -> 101 us with the clearing, 96 meshes of 1.4M
-// 194 -> 120 us, 460,000 vertices of which 2 % move 97 -> 65 us).
+// vertices inserted too (with the clearing: 1M vertices, all moving 125 -> 58 us, 2 % of
+// them 94 -> 40; 200,000 in one mesh 61 -> 31, in 64 meshes 97 -> 42).
 __device__ __forceinline__ unsigned fbits(float x) { return x == 0.f ? 0u : __float_as_uint(x); }
 
 __device__ __forceinline__ float2 cand_pos(const float2* pos, const float2* d, const unsigned char* vfix, int v) {
@@ -201,8 +201,16 @@ __global__ void __launch_bounds__(256) k_settle(SettleArgs A) {
   constexpr int U = kSettleUnroll;
   unsigned stamp = base + 1;
   bool lost = false;
+  // the mesh that this block has last stamped for the j-th vertices of its threads: without
+  // it the first wave's warps all stamp the few meshes there are (29,000 stores to one
+  // address, 60 us)
+  __shared__ int s_stamped[U];
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < U) s_stamped[threadIdx.x] = -1;
   if (gtid == 0) words[2] = 0;
-  for (int first = gtid; first < A.A.V_it; first += stride * U) {
+  __syncthreads();
+  for (int first0 = gtid - lane; first0 < A.A.V_it; first0 += stride * U) {
+    const int first = first0 + lane;
     int v[U], comp[U], holder[U];
     unsigned h[U];
     float2 p[U];
@@ -223,8 +231,12 @@ __global__ void __launch_bounds__(256) k_settle(SettleArgs A) {
       if (v[j] >= 0) holder[j] = atomicCAS(A.table + h[j], kNoVertex, v[j]);
 #pragma unroll
     for (int j = 0; j < U; ++j) {
-      if (v[j] < 0) continue;
-      if ((unsigned)ld_i(reinterpret_cast<const int*>(A.smove) + comp[j]) != stamp) __stcg(A.smove + comp[j], stamp);
+      const int c = v[j] >= 0 ? comp[j] : -1;
+      const unsigned same = __match_any_sync(0xffffffffu, c);
+      if (c >= 0 && __ffs((int)same) - 1 == lane && atomicExch(s_stamped + j, c) != c &&
+          (unsigned)ld_i(reinterpret_cast<const int*>(A.smove) + c) != stamp)
+        __stcg(A.smove + c, stamp);
+      if (c < 0) continue;
       unsigned it = 0;
       while (holder[j] != kNoVertex) {
         if (settle_same(A, holder[j], p[j], comp[j])) {
@@ -253,7 +265,7 @@ __global__ void __launch_bounds__(256) k_settle(SettleArgs A) {
       const bool fixed = A.vfix[v[j]] != 0;
       if (!fixed && (q.x != 0.f || q.y != 0.f)) continue;
       comp[j] = A.vcomp ? A.vcomp[v[j]] : 0;
-      if ((unsigned)ld_i(reinterpret_cast<const int*>(A.smove) + comp[j]) != stamp) continue;
+      if (A.smove[comp[j]] != stamp) continue;  // through L1: nothing is stamped any more
       p[j] = A.pos[v[j]];
       h[j] = settle_slot(p[j], comp[j], A.mask);
       holder[j] = ld_i(A.table + h[j]);
