@@ -2815,6 +2815,14 @@ __device__ __forceinline__ void star_marked(const KParams& P, unsigned cs, int i
 // A build most of whose stars still disagree after this many rounds is left to
 // insertion: the order said too little about who is near whom.
 constexpr int kStarSettling = 12;
+// So is one with a vertex that many others still tell of themselves after a few rounds: it
+// takes in kInbox - 1 of them a round, a lone thread's 100 us each, and more than 128
+// neighbours are no star.  Points on a circle around one, a whole build in us by insertion
+// alone, with the stars to their end, and so: 80 points 1050, 1680, 1050; 130 1180, 3750,
+// 1110; 1,000 1790, 5820, 1780.  (From 40 after two rounds on: 910, 1040 and 1510, but
+// 100,000 points of a Cauchy distribution 7.5 ms for 5.8.)
+constexpr int kStarWideRounds = 3;
+constexpr int kStarTold = 48;
 
 // Vertices (or list entries) per warp of the launch up to which a warp takes one
 // vertex at a time; above it a thread does.
@@ -2973,6 +2981,7 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
           const int v = base + lane < n ? ld_i(list + base + lane) : -1;
           int rc = kStarOk;
           if (v >= 0) {
+            if (kBuild && rounds > kStarWideRounds) fine = fine && ld_i(P.sinbox + (size_t)kInbox * v) < kStarTold;
             SharedCand L;
             rc = star_from_stars(P, v, L, lc);
           }
@@ -2986,6 +2995,7 @@ __device__ __forceinline__ bool star_step(cg::grid_group& g, const KParams& P, u
       } else {
         for (int i = gwarp; i < n; i += nwarps) {
           const int v = ld_i(list + i);
+          if (kBuild && rounds > kStarWideRounds) fine = fine && ld_i(P.sinbox + (size_t)kInbox * v) < kStarTold;
           warp_touch(P, v, ts);
           if (!warp_from_stars(P, v, lc) && lane == 0) fine = star_alone(P, v, false, 0, true, lc) && fine;
           __syncwarp();
