@@ -2759,6 +2759,10 @@ __device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, 
 //    more than kStarSparse vertices: 460,000 vertices of which 2 % move, stars 1117 us a
 //    pass, removal 800; 200,000 and below, stars 0.6 to 0.9 of removal at any number of
 //    movers;
+//  - few vertices moved, and far: each has turned more than two faces (six of their sides).
+//    A star finds its way one neighbour a round, removal walks.  3 x spacing, us by stars
+//    and by removal: 50,000 vertices, 150 movers 959 and 518; 512 meshes of 300, 460 movers
+//    730 and 470; but 1,000 vertices, 50 movers 324 and 420;
 //  - the mesh has more than kStarMost vertices.  Uniform points, sigma = 0.1 x spacing,
 //    stars and removal in ms: 1M 1.23 and 1.67, 2M 2.12 and 2.15, 2.5M 2.58 and 2.48, 3M
 //    3.12 and 2.92, 4M 4.06 and 3.29, 8.5M 8.34 and 6.05;
@@ -2779,15 +2783,18 @@ __device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, 
 //    Over 135 such steps of 500,000 to 2.5M vertices the rule's side is 0.3 % slower than
 //    the better one on average, 5 % slower than removal at most.
 constexpr int kStarSparse = 200000;
+constexpr int kStarNear = 4096;
 constexpr int kStarMost = 2500000;
 constexpr int kStarDense = 850000;   // open edges allowed: 0.28 a vertex above this
 constexpr int kStarTurned = 670000;  // the least vertices where a handful of turned faces goes to removal
 __device__ __forceinline__ bool removal_first(const KParams& P, int turned, bool sparse) {
   if (P.V_it > kStarMost || (sparse && P.V_it > kStarSparse)) return true;
+  if (P.V_it <= kStarNear) return false;
+  const long long movers = P.move_mode == MOVE_NONE ? P.V_it : ld_i(&P.st->movers_now);
+  if (16 * movers < P.V_it && turned > 6 * movers) return true;
   if (P.V_it <= kStarTurned) return false;
   const long long n = ld_i(&P.st->wl_count[0]);
   if (turned < 128 && 128 * n < P.V_it) return true;
-  const long long movers = P.move_mode == MOVE_NONE ? P.V_it : ld_i(&P.st->movers_now);
   const float open = 4 * movers < P.V_it ? 0.333f * (float)n : (32ll * turned < n ? 2.f : 1.f) * (float)n;
   return open < 0.28f * (float)(P.V_it - kStarDense);
 }

@@ -133,3 +133,21 @@ def test_neighbours_that_move_together_far(M, n, far):
         st, pos = step(b, pos, d.astype(np.float32))
         assert st["inverted_faces"] > 0 and st["lawson_flips"] == 0, st
     b.close()
+
+
+@pytest.mark.parametrize("n,movers,stars", [(3000, 20, True), (6000, 20, False), (40000, 400, False)])
+def test_few_that_move_far(M, n, movers, stars):
+    """A handful of vertices that jump several spacings go by removal, but in the smallest
+    meshes; the rest of the mesh does not move."""
+    b = M.MeshBatch.from_points([uniform_points(n, 5)])
+    pos = positions(b)
+    rng = np.random.default_rng(n)
+    d = np.zeros_like(pos)
+    m = rng.choice(np.arange(4, b.V), movers, replace=False)
+    d[m] = rng.uniform(200, 8000, (movers, 2)) - pos[m]
+    far = np.abs(d).max(1) > 8 * spacing(n)
+    d[far] *= 8 * spacing(n) / np.abs(d[far]).max(1)[:, None]
+    st, pos = step(b, pos, d)
+    assert st["inverted_faces"] > 6 * movers
+    assert (st["lawson_flips"] == 0) == stars
+    b.close()
