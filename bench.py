@@ -527,19 +527,71 @@ def run_ours(args, rank, world, dist):
             "predicate_errors": parity["sign_disagreements"] if parity else None,
             "parity": parity, "repair": repair, "batched": batched,
             "e2e": e2e, "cpu_baseline": cpu, "clocks": clocks,
-            # k_step per step, plus k_one_ring + 7 grid-build kernels + k_grid_frnn per step
-            "gpu_launches": K * (10 if do_q else 1),
+            # k_step per step, plus k_one_ring + 4 grid-build kernels (k_grid_hash, k_cell_scan,
+            # k_grid_bucket, k_grid_place) + k_grid_frnn per step
+            "gpu_launches": K * (7 if do_q else 1),
             "wall_s": wall, "build_s": t_build,
         }
         print(json.dumps(line), flush=True)
 
 
 # ---------------------------------------------------------------------------
+PHASES = {"stars": ("classify", "first_stars", "rounds", "number", "write", "tail"),
+          "removal": ("classify", "send_back", "remove", "reinsert", "lawson", "tail")}
+
+
+def untangle_record(tl, trm, tin, counters, stats):
+    """What one untangling step did, from the kernel's marks and counters: by stars or by
+    removal, the time between the marks of that way (us), its rounds, and the last of
+    them in detail."""
+    passes, removals = int(counters[14]), int(counters[15])
+    by = "removal" if removals > 0 else "stars"
+    marks = np.array([tl[0], tl[1], tl[43], tl[44], tl[45], tl[46], tl[47]], np.float64)
+    rec = {"by": by, "phases": np.diff(marks) / 1e3}
+    if by == "stars":
+        # the step counts one round more than the rounds of stars after the first
+        n = max(0, int(stats["insert_rounds"]) - 1)
+        ends = [int(tl[2 + r]) for r in range(min(n, 40))]
+        rec["rounds"] = {"stars": n}
+        rec["detail"] = {"round_us": [round((e - p) / 1e3, 1) for p, e in zip([int(tl[43])] + ends, ends)]}
+        return rec
+    rec["rounds"] = {"fixpoint_passes": passes, "removal": removals, "insertion": int(stats["insert_rounds"]),
+                     "flip": int(stats["lawson_rounds"])}
+
+    def split(prev, rows, end):
+        out = []
+        for r in rows:
+            out.append([round(float(y - x) / 1e3, 1) for x, y in zip([prev] + list(r[:2]), r[:3])])
+            prev = r[end]
+        return out
+
+    ends = [int(x) for x in trm[48:48 + min(passes, 16)]]
+    rec["detail"] = {
+        "send_back_pass_us": [round((e - p) / 1e3, 1) for p, e in zip([int(tl[1])] + ends, ends)],
+        "removal_round_us": split(tl[43], [trm[4 * r:4 * r + 4] for r in range(min(removals, 16))], 2),
+        "insertion_round_us": split(tl[44], [tin[4 * r:4 * r + 4] for r in range(min(int(stats["insert_rounds"]), 16))],
+                                    3),
+        "slowest_removal_cycles_spokes": [[int(x) >> 16, int(x) & 0xffff] for x in trm[64:64 + min(removals, 16)]],
+        "uncached_removals": [int(x) for x in trm[80:80 + min(removals, 16)]]}
+    return rec
+
+
+def untangle_bytes(V, E, stats, by):
+    """Algorithmic bytes of a step that untangles: the move and the classification, and by
+    removal the work-list items and flips after it.  (By stars every record is written
+    again, which is the form's own cost and not counted.)"""
+    base = 24 * V + 16 * E + 8 * V
+    if by == "stars":
+        return base
+    items = max(0, stats["incircle_tests"] - (E - 4))
+    return base + 20 * items + 96 * (stats["lawson_flips"] + stats["removal_flips"])
+
+
 def repair_measure(n, K, Wm, seed, local):
-    """The repair path at the headline size: an n-point mesh under a Gaussian
+    """Untangling at the headline size: an n-point mesh under a Gaussian
     random walk (sigma = 0.1 x mean spacing, clamped to the box, coincident
-    moves settled), which inverts faces every step, so every step runs the
-    untangle repair (send back, remove, Lawson, reinsert).  K timed steps of
+    moves settled), which inverts faces every step, so every step makes stars
+    anew or, where the engine chooses it, removes and reinserts.  K timed steps of
     k_step (CUDA events on its stream, L2 flushed before each), with the
     phase split from the kernel's own %globaltimer marks."""
     import ctypes as C
@@ -563,12 +615,11 @@ def repair_measure(n, K, Wm, seed, local):
             "insert_rounds", "lawson_rounds", "incircle_tests", "incircle_fp64", "incircle_exact", "orient_fp64",
             "orient_exact")
     tot = {k: 0 for k in keys}
-    ms, phases, rounds = [], [], []
+    ms, records, alg = [], [], 0
     tl = np.zeros(48, np.int64)
     cn = np.zeros(32, np.int64)
     trm = np.zeros(96, np.int64)
     tin = np.zeros(64, np.int64)
-    last_rounds = None
     for k in range(Wm + K):
         mesh.walk(sigma, counter, d, seed=77, stream=stream)
         mesh.settle(d, stream=stream)
@@ -590,61 +641,34 @@ def repair_measure(n, K, Wm, seed, local):
         for key in keys:
             tot[key] += sd[key]
         L.check(lib.mcl_debug_timeline(mesh.handle, L.ptr(tl)))
-        t0 = tl[0]
-        # start -> classified -> reverted -> removed -> reinserted -> Lawson -> end
-        marks = [tl[1], tl[43], tl[44], tl[45], tl[46], tl[47]]
-        phases.append(np.diff(np.array([t0] + marks, np.float64)) / 1e3)
         if lib.mcl_debug_counters(mesh.handle, L.ptr(cn), len(cn)) < 16:  # returns how many counters exist
             raise RuntimeError("mcl_debug_counters failed")
-        rounds.append((cn[14], cn[15], sd["insert_rounds"], sd["lawson_rounds"]))
-        # the last step's rounds: send-back passes, removal rounds (claim,
-        # verify, remove), insertion rounds (locate, win, split), in us
         L.check(lib.mcl_debug_remove_timeline(mesh.handle, L.ptr(trm)))
         L.check(lib.mcl_debug_insert_timeline(mesh.handle, L.ptr(tin)))
-        npass, nrem, nins = int(min(cn[14], 16)), int(min(cn[15], 16)), int(min(sd["insert_rounds"], 16))
-        prev = tl[1]
-        passes = []
-        for p_ in range(npass):
-            passes.append((trm[48 + p_] - prev) / 1e3)
-            prev = trm[48 + p_]
-        prev = tl[43]
-        rem = []
-        for r_ in range(nrem):
-            m3 = [trm[4 * r_], trm[4 * r_ + 1], trm[4 * r_ + 2]]
-            rem.append([round((m3[0] - prev) / 1e3, 1), round((m3[1] - m3[0]) / 1e3, 1), round((m3[2] - m3[1]) / 1e3, 1)])
-            prev = m3[2]
-        prev = tl[44]
-        ins = []
-        for r_ in range(nins):
-            m3 = [tin[4 * r_], tin[4 * r_ + 1], tin[4 * r_ + 2]]
-            ins.append([round((m3[0] - prev) / 1e3, 1), round((m3[1] - m3[0]) / 1e3, 1), round((m3[2] - m3[1]) / 1e3, 1)])
-            prev = tin[4 * r_ + 3]
-        last_rounds = {"send_back_pass_us": [round(x, 1) for x in passes], "removal_round_us": rem,
-                       "insertion_round_us": ins,
-                       "slowest_removal_cycles_spokes": [[int(trm[64 + r_]) >> 16, int(trm[64 + r_]) & 0xffff]
-                                                         for r_ in range(nrem)],
-                       "uncached_removals": [int(trm[80 + r_]) for r_ in range(nrem)]}
+        records.append(untangle_record(tl, trm, tin, cn, sd))
+        alg += untangle_bytes(V, E, sd, records[-1]["by"])
     ms = np.array(ms)
-    ph = np.median(np.array(phases), 0)
     flips = tot["lawson_flips"] + tot["removal_flips"]
-    wl_items = max(0, tot["incircle_tests"] - K * (E - 4))
-    alg = 24 * V + 16 * E + 8 * V + 20 * wl_items / K + 96 * flips / K
+    alg /= K
+    ways = {w: [r for r in records if r["by"] == w] for w in PHASES}
+    by = max(ways, key=lambda w: len(ways[w]))
+    of = ways[by]
+    ph = np.median(np.array([r["phases"] for r in of]), 0)
     peak, peak_kind = peaks()
     mesh.close()
     return {"workload": f"{n} points uniform, Gaussian random walk sigma = 0.1 x mean spacing (clamped, coincident "
-                        "moves settled); every step inverts faces and runs the repair",
+                        "moves settled); every step inverts faces and untangles them",
             "steps": K, "ms_per_step": float(ms.mean()), "p50_ms": float(np.median(ms)),
             "p99_ms": float(np.percentile(ms, 99)), "pts_steps_per_s": n * K / (ms.sum() / 1e3),
             "flips_per_s": flips / (ms.sum() / 1e3),
             "per_step": {k: tot[k] / K for k in keys},
-            "phase_us_median": {"classify": ph[0], "send_back": ph[1], "remove": ph[2], "reinsert": ph[3],
-                                "lawson": ph[4], "tail": ph[5]},
-            "rounds_median": dict(zip(("fixpoint_passes", "removal", "insertion", "flip"),
-                                      np.median(np.array(rounds), 0).tolist())),
-            "last_step_rounds": last_rounds,
+            "untangled_by": {w: len(r) for w, r in ways.items()},
+            "phase_us_median": dict(zip(PHASES[by], ph.tolist())),
+            "rounds_median": {k: float(np.median([r["rounds"][k] for r in of])) for k in of[-1]["rounds"]},
+            "last_step_rounds": of[-1]["detail"],
             "roofline": {"bound": "hbm", "achieved": alg / (ms.mean() / 1e3) / 1e9, "peak": peak,
                          "frac": alg / (ms.mean() / 1e3) / 1e9 / peak, "peak_kind": peak_kind,
-                         "alg_bytes_per_launch": alg, "kernel": "k_step (repair)"},
+                         "alg_bytes_per_launch": alg, "kernel": f"k_step ({by})"},
             "l2": "flushed (256 MB write) before every timed step"}
 
 
@@ -862,9 +886,8 @@ def run_batched(args, rank, world, dist):
                    "l2": "inputs larger than L2 (no flush)", "parallelism": f"replicas x{world}"},
         "clocks": clocks,
         # per step: k_walk + k_advance, k_settle, k_step, and the grid FRNN
-        # (k_bgrid_hash, 3 scan kernels, k_bgrid_scatter, k_grid_sort_cells,
-        # k_gather, k_bgrid_frnn)
-        "gpu_launches": args.steps * 12,
+        # (k_bgrid_hash, k_cell_scan, k_grid_bucket, k_grid_place, k_bgrid_frnn)
+        "gpu_launches": args.steps * 9,
     }
     line.update({k: v for k, v in r.items() if k not in ("kin_s", "steps", "warmup", "meshes", "points", "vertices",
                                                         "edges", "ms_per_step")})
@@ -1034,7 +1057,7 @@ def run_precision(args, rank, world, dist):
         "totals": tot, "settled_moves": settled,
         "sign_check": "tests/test_gpu_precision.py compares sampled live-mesh predicate signs with the exact oracle",
         "step_ms": {"p50": float(np.median(ms)), "p99": float(np.percentile(ms, 99))},
-        "clocks": clocks, "gpu_launches": K * 5, "build_s": t_build,
+        "clocks": clocks, "gpu_launches": K * 4, "build_s": t_build,
     }
     if rank == 0:
         print(json.dumps(line), flush=True)
