@@ -2136,23 +2136,9 @@ __device__ __noinline__ int send_back(cg::grid_group g, const KParams P, unsigne
 
 // The rest of it: remove the vertices sent back (fs), reinsert them at the new positions,
 // Lawson.  Out of line, so k_step's hot loops keep their registers; keeps its own
-// counters and returns the next free stamp.  fs = 0: nothing has been sent back yet, or a
-// send-back was given up.
+// counters and returns the next free stamp.
 __device__ __noinline__ unsigned repair_step(cg::grid_group g, const KParams P, unsigned stamp, unsigned q0,
                                              unsigned fs) {
-  if (fs == 0) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      for (int i = 0; i < 3; ++i) P.st->fix_new[i] = P.st->fix_bad[i] = P.st->fix_list[i] = 0;
-      P.st->fix_all = 0;
-    }
-    g.sync();
-    fs = stamp++;
-    const int rc = send_back(g, P, fs, LLONG_MAX);
-    if (rc != MCL_OK) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) set_error(P, rc);
-      return stamp;
-    }
-  }
   LocalCounters lc = {0, 0, 0, 0, 0, 0, 0};
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
   KParams Q = P;
@@ -3116,25 +3102,41 @@ __global__ void __launch_bounds__(kThreads, 3) k_step(const __grid_constant__ KP
     // no stars where sub-steps are asked for, on a mesh that is not its square's, and for
     // a while after they could not be made
     const bool never = P.substeps > 0 || !P.square, held = hold > 0;
-    const unsigned fs = stamp++;
+    if (first && held) P.st->star_tried = kStarsHeld;
+    // A send-back, unless stars go first; stars, if it is given up; and a send-back to its
+    // end, if they cannot be made.  One call of each: with two, removal and the stars both
+    // lost registers (512 meshes of 8.5M vertices 8.2 -> 8.6 ms, 1M random walkers 1233 ->
+    // 1252 us).
+    bool stars = !(never || held || removal_first(P, inverted, sparse)), done = false;
+    long long most = never ? LLONG_MAX : 2ll * inverted + kSentBack;
+    unsigned fs = stamp++;
     int rc = kSentBackMany;
-    if (never || held || removal_first(P, inverted, sparse))
-      rc = send_back(g, P, fs, never ? LLONG_MAX : 2ll * inverted + kSentBack);
-    if (rc == MCL_OK || never) {
-      if (first && held) P.st->star_tried = kStarsHeld;
-      if (rc == MCL_OK) stamp = repair_step(g, P, stamp, q0, fs);
-      else if (first) set_error(P, rc);
-    } else {
-      // Nothing lives over the send-back's call that the stars need: the counters are
-      // flushed and the stamps read again, which keeps registers for the loops of
-      // star_step (1M random walkers 1265 -> 1245 us).
+    for (;;) {
+      if (!stars) {
+        rc = send_back(g, P, fs, most);
+        if (rc == MCL_OK || most == LLONG_MAX) break;
+        g.sync();  // its counts have been read; the next barrier is the stars'
+        if (first) {
+          for (int i = 0; i < 3; ++i) P.st->fix_new[i] = P.st->fix_bad[i] = P.st->fix_list[i] = 0;
+          P.st->fix_all = 0;
+        }
+      }
+      // Nothing lives over these calls that the stars need: the counters are flushed and
+      // the stamps read again.
       flush_counters(P, lc);
       lc = LocalCounters{0, 0, 0, 0, 0, 0, 0};
       const unsigned q = s_q0;
       stamp = q + 3;  // q, q + 1 and fs are taken
-      const bool done = star_step<false>(g, P, stamp, q, q + 1, lc);
+      done = star_step<false>(g, P, stamp, q, q + 1, lc);
       if (blockIdx.x == 0 && threadIdx.x == 0) P.st->star_tried = done ? kStarsMade : kStarsFailed;
-      if (!done) stamp = repair_step(g, P, stamp, q, 0);
+      if (done) break;
+      stars = false;
+      most = LLONG_MAX;
+      fs = stamp++;
+    }
+    if (!done) {
+      if (rc == MCL_OK) stamp = repair_step(g, P, stamp, s_q0, fs);
+      else if (blockIdx.x == 0 && threadIdx.x == 0) set_error(P, rc);
     }
   }
   flush_counters(P, lc);
