@@ -37,7 +37,8 @@
 // set of 500,000 (a third of it in clusters that move 1.4 of their spacings) 3332 ->
 // 2130 us.
 //
-// The bodies are host/device code: the CPU can run them vertex by vertex.
+// The bodies are host/device code: tests/cpp/star_rounds.cu runs them vertex by vertex
+// on the CPU.
 #pragma once
 
 #include "engine.cuh"
