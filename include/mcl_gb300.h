@@ -330,7 +330,8 @@ int mcl_mesh_clone(const mcl_mesh* src, mcl_mesh** out);
  * either.  mcl_mesh_get_tuning gives the values in use; setting them again
  * changes nothing. */
 int mcl_mesh_set_tuning(mcl_mesh* m, int blocks_per_sm, int tail_items);
-/* Work-list tile of the repair's removal rounds: how many lanes of each warp
+/* Work-list tile of the rounds of removal, where a step goes that way (few movers
+ * of a large mesh, the largest meshes, sub-steps): how many lanes of each warp
  * take entries of the vertex list (1..32; 0 = automatic, as few as let one
  * pass over the grid take the list).  A removal is a long divergent chain,
  * so fewer lanes per warp run faster when the grid has warps to spare.
@@ -338,8 +339,9 @@ int mcl_mesh_set_tuning(mcl_mesh* m, int blocks_per_sm, int tail_items);
 int mcl_mesh_set_removal_tile(mcl_mesh* m, int tile);
 int mcl_mesh_get_removal_tile(const mcl_mesh* m, int* tile);
 
-/* Repair sub-steps per kinetic step (default 0: every vertex sent back while
- * untangling is removed and reinserted at its target).  A sub-step moves the
+/* Repair sub-steps per kinetic step (default 0: untangling makes stars anew, or
+ * removes and reinserts every vertex sent back, whichever is the faster).  With
+ * sub-steps vertices are always sent back first.  A sub-step moves the
  * sent-back vertices toward their targets as far as their stars allow and
  * restores the Delaunay property around them; those still short of their
  * targets after the last sub-step are removed and reinserted.  The resulting

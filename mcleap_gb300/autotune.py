@@ -7,8 +7,8 @@ speed but never its result:
   of the grid-wide barriers of the flip rounds);
 * the work-list size at or below which a single block finishes the flip rounds
   (block barriers instead of grid barriers for the long tail of small rounds);
-* the removal tile: how many lanes of a warp take entries of the repair's
-  vertex lists (its removals are long divergent chains).
+* the removal tile: how many lanes of a warp take entries of the vertex lists
+  of removal (long divergent chains); steps that untangle by stars do not use it.
 
 The first two are searched jointly, then the tile at the best pair.  Each
 candidate runs on a fresh clone of the mesh, so every candidate steps the same

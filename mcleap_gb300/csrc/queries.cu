@@ -914,8 +914,8 @@ __global__ void k_scan_add(int* out, const int* block_prefix, int64_t n) {
 // (coalesced), ids and rows mapped through src when given; what does not fit goes
 // straight to global memory.
 // Bound by the latency of the candidates' loads (some 50 per point at r = 1.92 cells of
-// 2.4 points): rows of 16 bits leave the L1 twice the room and let 40 warps reside
-// instead of 32, and both coordinates of a candidate share an instruction.  r = 3 x
+// 2.4 points): rows of 16 bits leave the L1 twice the room and let 48 warps reside
+// instead of 32 (41 are active on average), and both coordinates of a candidate share an instruction.  r = 3 x
 // spacing, 1,000,000 points, periodic: 176 -> 131 us (rows of 32 bits: 174).
 constexpr int kStageCap = 48;
 constexpr int kFrnnThreads = 128;

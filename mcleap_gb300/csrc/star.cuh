@@ -30,12 +30,12 @@
 //
 // What bounds it: below some ten thousand vertices the latency of one vertex's
 // dependent loads and tests and five to ten grid barriers; above, instruction issue
-// (about 180 warp instructions per vertex and star with 12 of 32 lanes at work: rings
-// and candidate lists differ in length) and L2 latency.  The step's launch at sigma =
-// 0.1 x spacing, removal path before -> stars, GB300: 1,000 points 472 -> 92 us,
-// 10,000 points 586 -> 155 us, 1,000,000 points 1551 -> 1260 us; the precision-stress
-// set of 500,000 (a third of it in clusters that move 1.4 of their spacings) 3332 ->
-// 2130 us.
+// (456 warp instructions per vertex of a 1M-point step, with 12.6 of 32 lanes at work:
+// rings and candidate lists differ in length), barriers and L2 latency.  A step at sigma =
+// 0.1 x spacing, from the call to its record, by removal -> by stars, GB300: 1,000 points
+// 460 -> 110 us, 10,000 points 610 -> 185 us, 500,000 points 1290 -> 780 us, 1,000,000
+// points 1640 -> 1230 us; a pass of the precision-stress set of 500,000 (a third of it in
+// clusters that move 1.4 of their spacings) 2860 -> 1860 us.
 //
 // The bodies are host/device code: tests/cpp/star_rounds.cu runs them vertex by vertex
 // on the CPU.
