@@ -2746,10 +2746,20 @@ __device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, 
 //    more than kStarSparse vertices: 460,000 vertices of which 2 % move, stars 1117 us a
 //    pass, removal 800; 200,000 and below, stars 0.6 to 0.9 of removal at any number of
 //    movers;
-//  - few vertices moved, and far: each has turned more than two faces (six of their sides).
-//    A star finds its way one neighbour a round, removal walks.  3 x spacing, us by stars
-//    and by removal: 50,000 vertices, 150 movers 959 and 518; 512 meshes of 300, 460 movers
-//    730 and 470; but 1,000 vertices, 50 movers 324 and 420;
+//  - few vertices moved (a sixteenth, or an eighth of more than kStarFar), and far: each has
+//    turned more than two faces (six of their sides), fewer in larger meshes.  A star finds
+//    its way one neighbour a round, removal walks.  us by stars and by removal: 50,000
+//    vertices, 150 movers by 3 x spacing 959 and 518; 512 meshes of 300, 460 movers by 3 x
+//    730 and 470; 175,000 vertices, 500 movers by 1.5 x 1362 and 498; 64 meshes of 3,000,
+//    600 movers by 1 x 486 and 410; but 1,000 vertices, 50 movers by 3 x 324 and 420;
+//  - up to six sevenths moved, and far: most of the faces with a moved corner turned.  The
+//    line is on turned sides a face, the faces with a mover counted as 1 - (1 - movers)^3 of
+//    two a vertex; it rises with the movers, as removal then walks among more holes, and
+//    falls as the mesh grows.  us by stars and by removal: 195,000 vertices, 25 % by 2 x
+//    spacing 2230 and 1640, 45 % by 2 x 2490 and 2000, 70 % by 3 x 4340 and 2830, but 70 % by
+//    1 x 1590 and 2280, all by 2 x 2980 and 4450; 64 meshes of 3,000, 10 % by 2 x 1460 and
+//    943; 600,000, 45 % by 2 x 5580 and 3680; 50,000, 45 % by 3 x 1950 and 1590, by 2 x 1314
+//    and 1490.  20,000 vertices are within 14 % of removal by 3 x and further, and gain below;
 //  - the mesh has more than kStarMost vertices.  Uniform points, sigma = 0.1 x spacing,
 //    stars and removal in ms: 1M 1.23 and 1.67, 2M 2.12 and 2.15, 2.5M 2.58 and 2.48, 3M
 //    3.12 and 2.92, 4M 4.06 and 3.29, 8.5M 8.34 and 6.05;
@@ -2772,6 +2782,7 @@ __device__ __forceinline__ void star_list(const KParams& P, int u, unsigned cs, 
 //    a swarm in one place (1M vertices, 1,400 faces: 678 by stars, 814).
 constexpr int kStarSparse = 200000;
 constexpr int kStarNear = 4096;
+constexpr int kStarFar = 100000;
 constexpr int kStarMost = 2500000;
 constexpr int kStarDense = 850000;   // open edges allowed: 0.28 a vertex above this
 constexpr int kStarTurned = 670000;  // the least vertices where a handful of turned faces goes to removal
@@ -2779,7 +2790,13 @@ __device__ __forceinline__ bool removal_first(const KParams& P, int turned, bool
   if (P.V_it > kStarMost || (sparse && P.V_it > kStarSparse)) return true;
   if (P.V_it <= kStarNear) return false;
   const long long movers = P.move_mode == MOVE_NONE ? P.V_it : ld_i(&P.st->movers_now);
-  if (16 * movers < P.V_it && turned > 6 * movers) return true;
+  const bool wide = P.V_it > kStarFar, few = 16 * movers < P.V_it || (wide && 8 * movers < P.V_it);
+  if (few && turned > (wide ? 3 : P.V_it > kStarFar / 3 ? 5 : 6) * movers) return true;
+  if (!few && P.V_it > kStarFar / 3 && 7 * movers < 6ll * P.V_it) {
+    const float m = (float)movers / (float)P.V_it, still = (1.f - m) * (1.f - m) * (1.f - m);
+    const float far = !wide ? 2.f + 0.9f * m : P.V_it <= 5 * kStarFar / 2 ? 1.6f + 1.2f * m : 1.f + 1.6f * m;
+    if ((float)turned > far * (1.f - still) * (float)P.V_it) return true;
+  }
   if (P.V_it <= kStarTurned) return false;
   const long long n = ld_i(&P.st->wl_count[0]);
   if (turned < 128 && 128 * n < P.V_it) return true;

@@ -151,3 +151,18 @@ def test_few_that_move_far(M, n, movers, stars):
     assert st["inverted_faces"] > 6 * movers
     assert (st["lawson_flips"] == 0) == stars
     b.close()
+
+
+@pytest.mark.parametrize("n,part,far,stars", [
+    (20000, 0.45, 3.0, True), (40000, 0.45, 1.0, True), (40000, 0.45, 4.0, False), (40000, 1.0, 2.0, True),
+    (120000, 0.1, 3.0, False), (120000, 0.3, 1.0, True), (120000, 0.7, 4.0, False), (300000, 0.45, 2.0, False)])
+def test_some_that_move_far(M, n, part, far, stars):
+    """A part of the vertices moves several spacings while the rest stays: removal once
+    most of the faces that have a mover are turned."""
+    b = M.MeshBatch.from_points([uniform_points(n, 6)])
+    pos = positions(b)
+    d = gaussian_disp(len(pos), far * spacing(n), 7, pos)
+    d[np.random.default_rng(8).random(len(d)) >= part] = 0
+    st, pos = step(b, pos, d)
+    assert (st["lawson_flips"] == 0) == stars, st
+    b.close()
